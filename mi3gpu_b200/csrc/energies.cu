@@ -104,24 +104,21 @@ __device__ __forceinline__ void energies_chunk(const float *js, const uint32_t *
 }
 
 // Full slices with lanes over pairs (tiling.cuh): the table is [cell][P];
-// lane w visits pair (t + w) mod P at step t.  Each sequence's B*B terms are
-// summed as B float partial sums (step rows th, at most B terms each) added
-// in double, then in fixed point as above.
+// each lane visits the pairs in its own rotated order.  Each sequence's B*B
+// terms are summed as B float partial sums (one per site row, B terms each)
+// added in double, then in fixed point as above.
 template <int B>
-__device__ __forceinline__ double lane_energy(uint32_t jbase, const uint32_t (&row)[B], const uint32_t (&col)[B],
-                                              uint32_t wl) {
+__device__ __forceinline__ double lane_energy(uint32_t jbase, const uint32_t (&row)[B], const uint32_t (&col)[B]) {
     float part[B];
 #pragma unroll
     for (int th = 0; th < B; ++th) part[th] = 0.0f;
 #pragma unroll
     for (int tl = 0; tl < B; ++tl) {
-        const bool carry = tl + wl >= (uint32_t)B;
         const uint32_t c = jbase + col[tl];
 #pragma unroll
         for (int th = 0; th < B; ++th) {
-            const uint32_t r = carry ? row[(th + 1) & (B - 1)] : row[th];
             float v;
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(c + r));
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(c + row[th]));
             part[th] += v;
         }
     }
@@ -136,7 +133,7 @@ __device__ __forceinline__ void energies_chunk_lanes(const float *js, const uint
                                                      uint32_t nbeg, uint32_t nend, unsigned long long *acc,
                                                      uint32_t L, uint32_t q, uint32_t bi, uint32_t bj) {
     const uint32_t swords = (L - 1) / 4 + 1;
-    const uint32_t lane = threadIdx.x & 31, wl = lane % B;
+    const uint32_t lane = threadIdx.x & 31;
     const uint32_t jbase = (uint32_t)__cvta_generic_to_shared(js);
     if constexpr (B == 16) {
         // 256 terms per sequence: one sequence per thread has loads enough
@@ -147,7 +144,7 @@ __device__ __forceinline__ void energies_chunk_lanes(const float *js, const uint
             load_block_words<B>(seq, buflen, n, bj, swords, wJ);
             uint32_t row[B], col[B];
             lane_offsets<B>(wI, wJ, q, lane, row, col);
-            const double e1 = lane_energy<B>(jbase, row, col, wl);
+            const double e1 = lane_energy<B>(jbase, row, col);
             atomicAdd(&acc[n], (unsigned long long)__double2ll_rn(e1 * FIX_SCALE));
         }
         return;
@@ -163,9 +160,9 @@ __device__ __forceinline__ void energies_chunk_lanes(const float *js, const uint
         load_block_words<B>(seq, buflen, two ? n2 : n, bj, swords, vJ);
         uint32_t row[B], col[B];
         lane_offsets<B>(wI, wJ, q, lane, row, col);
-        const double e1 = lane_energy<B>(jbase, row, col, wl);
+        const double e1 = lane_energy<B>(jbase, row, col);
         lane_offsets<B>(vI, vJ, q, lane, row, col);
-        const double e2 = lane_energy<B>(jbase, row, col, wl);
+        const double e2 = lane_energy<B>(jbase, row, col);
         atomicAdd(&acc[n], (unsigned long long)__double2ll_rn(e1 * FIX_SCALE));
         if (two) atomicAdd(&acc[n2], (unsigned long long)__double2ll_rn(e2 * FIX_SCALE));
     }
@@ -245,7 +242,7 @@ __global__ void k_energies_final(const unsigned long long *__restrict__ acc, flo
 template <int B, bool CONS>
 static int launch_energies(const float *J, const uint32_t *seq, uint32_t buflen, uint32_t nseq,
                            unsigned long long *acc, uint32_t L, uint32_t q, const uint8_t *cons, cudaStream_t st) {
-    SliceGeom g = make_geom(L, B, nseq, 148 * 8, 2048);
+    SliceGeom g = make_geom(L, B, nseq);
     size_t smem = (size_t)B * B * q * q * 4;
     cudaFuncSetAttribute(k_energies<B, CONS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     uint64_t nblk = (uint64_t)g.nslices * g.nchunks;

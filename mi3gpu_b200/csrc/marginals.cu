@@ -122,21 +122,18 @@ __device__ __forceinline__ void hist_chunk(uint32_t *h, const uint32_t *__restri
 }
 
 // Full slices with lanes over pairs (tiling.cuh): the histograms are
-// [cell][P]; lane w adds to pair (t + w) mod P at step t, so the 32 lanes of
-// a shared-memory reduction always hit 32 different banks and different
-// bins (no serialised same-bin adds either).
+// [cell][P] and each lane visits the pairs in its own rotated order, so the
+// 32 lanes of a shared-memory reduction always hit 32 different banks and
+// different bins (no serialised same-bin adds either).
 template <int B>
 __device__ __forceinline__ void lane_hist(uint32_t hbase, const uint32_t (&row)[B], const uint32_t (&col)[B],
-                                          uint32_t wl, uint32_t inc) {
+                                          uint32_t inc) {
 #pragma unroll
     for (int tl = 0; tl < B; ++tl) {
-        const bool carry = tl + wl >= (uint32_t)B;
         const uint32_t c = hbase + col[tl];
 #pragma unroll
-        for (int th = 0; th < B; ++th) {
-            const uint32_t r = carry ? row[(th + 1) & (B - 1)] : row[th];
-            asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(c + r), "r"(inc));
-        }
+        for (int th = 0; th < B; ++th)
+            asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(c + row[th]), "r"(inc));
     }
 }
 
@@ -145,7 +142,7 @@ __device__ __forceinline__ void hist_chunk_lanes(uint32_t *h, const uint32_t *__
                                                  uint32_t nbeg, uint32_t nend, const float *__restrict__ weights,
                                                  float scale, uint32_t L, uint32_t q, uint32_t bi, uint32_t bj) {
     const uint32_t swords = (L - 1) / 4 + 1;
-    const uint32_t lane = threadIdx.x & 31, wl = lane % B;
+    const uint32_t lane = threadIdx.x & 31;
     const uint32_t hbase = (uint32_t)__cvta_generic_to_shared(h);
     if constexpr (B == 16) {
         for (uint32_t n = nbeg + threadIdx.x; n < nend; n += blockDim.x) {
@@ -156,7 +153,7 @@ __device__ __forceinline__ void hist_chunk_lanes(uint32_t *h, const uint32_t *__
             if constexpr (WEIGHTED) inc = __float2uint_rn(__ldg(&weights[n]) * scale);
             uint32_t row[B], col[B];
             lane_offsets<B>(wI, wJ, q, lane, row, col);
-            lane_hist<B>(hbase, row, col, wl, inc);
+            lane_hist<B>(hbase, row, col, inc);
         }
         return;
     }
@@ -175,9 +172,9 @@ __device__ __forceinline__ void hist_chunk_lanes(uint32_t *h, const uint32_t *__
         }
         uint32_t row[B], col[B];
         lane_offsets<B>(wI, wJ, q, lane, row, col);
-        lane_hist<B>(hbase, row, col, wl, inc1);
+        lane_hist<B>(hbase, row, col, inc1);
         lane_offsets<B>(vI, vJ, q, lane, row, col);
-        lane_hist<B>(hbase, row, col, wl, two ? inc2 : 0u);
+        lane_hist<B>(hbase, row, col, two ? inc2 : 0u);
     }
 }
 
@@ -296,14 +293,17 @@ __global__ void k_chunks_to_float(const uint32_t *__restrict__ part, uint32_t nc
 
 constexpr uint32_t WMARG_CHUNK = 65536;  // sequences per CTA (fixed-point headroom)
 
+// The weighted chunk also sets the fixed-point scale (fixed_shift), so it is
+// never longer than what about 8 CTAs per SM would give, nor than
+// WMARG_CHUNK; each chunk costs a plane of bins, written and read once (the
+// larger overhead).
 template <int B, bool WEIGHTED>
 static SliceGeom pairhist_geom(uint32_t L, uint32_t nseq) {
-    SliceGeom g = make_geom(L, B, nseq, 148 * 8, 2048);
-    if (WEIGHTED && g.chunk > WMARG_CHUNK) {
-        g.chunk = WMARG_CHUNK;
-        g.nchunks = (nseq + g.chunk - 1) / g.chunk;
-    }
-    return g;
+    if (!WEIGHTED) return make_geom(L, B, nseq);
+    const uint32_t nb = (L + B - 1) / B, nslices = nb * (nb + 1) / 2;
+    const uint32_t want = (148 * 8 + nslices - 1) / nslices;
+    const uint32_t longest = (std::max<uint32_t>((nseq + want - 1) / want, 2048) + 255) & ~255u;
+    return make_geom(L, B, nseq, std::min(longest, WMARG_CHUNK), 2 * PAIR_CTA_OVERHEAD);
 }
 
 // Per-site residue sums over blocks of at most per_cta sequences (<= the pair

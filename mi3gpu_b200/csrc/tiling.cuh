@@ -48,18 +48,40 @@ inline uint32_t pick_block(uint32_t q, size_t budget, uint32_t max_b = 32) {
     return 0;
 }
 
-inline SliceGeom make_geom(uint32_t L, uint32_t B, uint32_t nseq, uint32_t target_ctas,
-                           uint32_t min_chunk) {
+// Chunk length by a wave model: nslices * nchunks CTAs run 2 per SM, so the
+// time goes as ceil(CTAs / 296) * (chunk + overhead), where staging and
+// flushing a slice's table costs about as much as PAIR_CTA_OVERHEAD sequences.
+// (Targeting a fixed number of CTAs instead left last waves nearly empty:
+// 2080 CTAs = 7.03 waves at L=512, q=21, 2^18 sequences.)
+// For each number of waves only the largest nchunks that fits it is tried,
+// from PAIR_MIN_WAVES on: slices differ in cost, which several CTAs per slot
+// even out.
+constexpr uint32_t PAIR_RESIDENT = 148 * 2, PAIR_CTA_OVERHEAD = 2048, PAIR_MIN_CHUNK = 1024, PAIR_MIN_WAVES = 3;
+
+inline SliceGeom make_geom(uint32_t L, uint32_t B, uint32_t nseq, uint32_t max_chunk = 0xffffff00u,
+                           uint32_t overhead = PAIR_CTA_OVERHEAD) {
     SliceGeom g;
     g.B = B;
     g.nb = (L + B - 1) / B;
     g.nslices = g.nb * (g.nb + 1) / 2;
-    uint32_t want = std::max<uint32_t>(1, (target_ctas + g.nslices - 1) / g.nslices);
-    uint32_t chunk = (nseq + want - 1) / want;
-    chunk = std::max(chunk, min_chunk);
-    chunk = (chunk + 255) & ~255u;
-    g.chunk = chunk;
-    g.nchunks = (nseq + chunk - 1) / chunk;
+    const uint32_t min_chunk = std::min(PAIR_MIN_CHUNK, max_chunk);
+    const uint32_t least = (nseq - 1) / max_chunk + 1;  // chunks that max_chunk asks for
+    const uint32_t most = std::max(least, (nseq - 1) / min_chunk + 1);
+    auto chunk_of = [&](uint32_t nc) { return std::min(max_chunk, ((nseq - 1) / nc + 1 + 255) & ~255u); };
+    g.chunk = chunk_of(least);
+    uint64_t best = ~0ull;
+    const uint32_t w0 = (uint32_t)(((uint64_t)g.nslices * least + PAIR_RESIDENT - 1) / PAIR_RESIDENT);
+    for (uint32_t w = std::max(w0, PAIR_MIN_WAVES); w < w0 + 24; ++w) {
+        const uint64_t fit = (uint64_t)w * PAIR_RESIDENT / g.nslices;
+        const uint32_t chunk = chunk_of((uint32_t)std::min<uint64_t>(std::max<uint64_t>(fit, least), most));
+        const uint64_t cost = w * ((uint64_t)chunk + overhead);
+        if (cost < best) {
+            best = cost;
+            g.chunk = chunk;
+        }
+        if (fit >= most) break;
+    }
+    g.nchunks = (nseq - 1) / g.chunk + 1;
     return g;
 }
 
@@ -137,15 +159,18 @@ __device__ __forceinline__ uint32_t slice_row(const uint32_t (&wI)[B / 4], int i
 // all visit pair p at the same time and gather 32 random cells: about 3.3
 // shared-memory wavefronts per warp instruction.  For full slices (every
 // pair valid) the pair kernels can instead lay the table out cell-major,
-// [cell][p] with P = B*B pairs (p = ii*B + jj), and let lane w visit pair
-// (t + w) mod P at step t: 32 consecutive pairs, 32 different banks, one
-// wavefront.  Lane w = B*wh + wl then meets pair (ii, jj) with
-// jj = (tl + wl) mod B and ii = (th + wh + carry) mod B for step
-// t = B*th + tl, carry = (tl + wl >= B).  Rotating the sequence's residue
-// bytes of block I by wh and of block J by wl (byte k of the rotated block
-// = byte (k + r) mod B) turns these into static register indices: the
-// column offset of step t is col[tl], the row offset row[th] or
-// row[th + 1] -- one select per pair.  P >= 32 needs B >= 8.
+// [cell][p] with P = B*B pairs (p = ii*B + jj).  Lane w = B*wh + wl visits, at
+// step (th, tl), the pair ii = (th + wh) mod B, jj = (tl + wl) mod B.  Its bank
+// is (ii*B + jj) mod 32: the B lanes of one wh hold B different jj, and the
+// 32/B values of wh hold ii that differ mod 32/B, so the 32 lanes use 32
+// different banks at every step -- one wavefront.  Rotating the sequence's
+// residue bytes of block I by wh and of block J by wl (byte k of the rotated
+// block = byte (k + r) mod B) makes the offsets static register indices: one
+// add, row[th] + col[tl], per pair.  (Visiting pair (t + w) mod P instead
+// needs a select per pair where t + w carries into the next row, on the
+// half-rate ALU: a Newton phase of 3 steps at L=232, q=21, 2^20 -- four energy
+// passes, a count and three weighted passes -- took 44.3 ms that way, 38.6 ms
+// this way.)  B >= 8.
 
 // byte k of o = byte (k + r) mod B of w, for 0 <= r < B
 template <int B>
