@@ -274,9 +274,9 @@ uint32_t mi3_bicounts_tc_plan(uint32_t L, uint32_t q, uint32_t nseq, uint32_t *o
 int mi3_bicounts_to_bimarg(const uint32_t *bicount, float *bimarg, uint32_t nseq, uint32_t L,
                            uint32_t q, void *stream);
 
-/* Bytes of workspace mi3_weighted_marg needs for nseq sequences:
- * 256 + 8*L*q (padded to 256) + 4 * nPairs * q*q per chunk of up to 65536
- * sequences. */
+/* Bytes of workspace mi3_weighted_marg needs for up to nseq sequences (never
+ * less for more): 256 + 8*L*q (padded to 256) + 4 * nPairs * q*q per chunk,
+ * chunks of 1024 to 65536 sequences. */
 size_t mi3_weighted_marg_workspace(uint32_t L, uint32_t q, uint32_t nseq);
 
 /* weightedMarg (mcmc.cl:646-718), MCMCGPU.weightedMarg (mcmcGPU.py:634-661):

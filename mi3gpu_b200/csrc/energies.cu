@@ -13,7 +13,7 @@
 // mcmc.cl:249-336); this result is at least as accurate.
 #include <mutex>
 
-#include "tiling.cuh"
+#include "joint.cuh"
 
 namespace mi3 {
 
@@ -103,69 +103,103 @@ __device__ __forceinline__ void energies_chunk(const float *js, const uint32_t *
     }
 }
 
-// Full slices with lanes over pairs (tiling.cuh): the table is [cell][P];
-// each lane visits the pairs in its own rotated order.  Each sequence's B*B
-// terms are summed as B float partial sums (one per site row, B terms each)
-// added in double, then in fixed point as above.
+// (hi, lo) floats += (hi, lo) floats: two independent float adds.
+__device__ __forceinline__ void add_f32x2(unsigned long long &acc, float lo, float hi) {
+    asm("{\n\t.reg .b64 v;\n\tmov.b64 v, {%1, %2};\n\tadd.rn.f32x2 %0, %0, v;\n\t}" : "+l"(acc) : "f"(lo), "f"(hi));
+}
+
+// One sequence's B*B terms, lanes over pairs: B float partial sums (one per
+// joint row, B terms each; two rows share a packed add), added in double.
 template <int B>
 __device__ __forceinline__ double lane_energy(uint32_t jbase, const uint32_t (&row)[B], const uint32_t (&col)[B]) {
-    float part[B];
+    unsigned long long part[B / 2];
 #pragma unroll
-    for (int th = 0; th < B; ++th) part[th] = 0.0f;
+    for (int th = 0; th < B / 2; ++th) part[th] = 0;
 #pragma unroll
     for (int tl = 0; tl < B; ++tl) {
         const uint32_t c = jbase + col[tl];
 #pragma unroll
-        for (int th = 0; th < B; ++th) {
-            float v;
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(c + row[th]));
-            part[th] += v;
+        for (int th = 0; th < B / 2; ++th) {
+            float v0, v1;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v0) : "r"(c + row[2 * th]));
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v1) : "r"(c + row[2 * th + 1]));
+            add_f32x2(part[th], v0, v1);
         }
     }
     double e = 0.0;
 #pragma unroll
-    for (int th = 0; th < B; ++th) e += (double)part[th];
+    for (int th = 0; th < B / 2; ++th) {
+        e += (double)__uint_as_float((uint32_t)part[th]);
+        e += (double)__uint_as_float((uint32_t)(part[th] >> 32));
+    }
     return e;
 }
 
-template <int B>
-__device__ __forceinline__ void energies_chunk_lanes(const float *js, const uint32_t *__restrict__ seq, uint32_t buflen,
-                                                     uint32_t nbeg, uint32_t nend, unsigned long long *acc,
-                                                     uint32_t L, uint32_t q, uint32_t bi, uint32_t bj) {
-    const uint32_t swords = (L - 1) / 4 + 1;
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t jbase = (uint32_t)__cvta_generic_to_shared(js);
-    if constexpr (B == 16) {
-        // 256 terms per sequence: one sequence per thread has loads enough
-        // in flight (16 independent partial sums) and fits the registers
-        for (uint32_t n = nbeg + threadIdx.x; n < nend; n += blockDim.x) {
-            uint32_t wI[B / 4], wJ[B / 4];
-            load_block_words<B>(seq, buflen, n, bi, swords, wI);
-            load_block_words<B>(seq, buflen, n, bj, swords, wJ);
-            uint32_t row[B], col[B];
-            lane_offsets<B>(wI, wJ, q, lane, row, col);
-            const double e1 = lane_energy<B>(jbase, row, col);
-            atomicAdd(&acc[n], (unsigned long long)__double2ll_rn(e1 * FIX_SCALE));
+// Energies over joint sites (joint.cuh).  Bound by instruction issue at two
+// per gather (an add and a load) plus the sequence's offsets, with the
+// shared-memory pipe close behind; figures in joint.cuh.
+template <int B, int GI, int GJ, int T>
+__global__ void __launch_bounds__(T, 1024 / T) k_energies_joint(const float *__restrict__ J,
+                                                               const uint32_t *__restrict__ seq, uint32_t buflen,
+                                                               uint32_t nseq, unsigned long long *acc, uint32_t L,
+                                                               uint32_t q, JointGeom g) {
+    extern __shared__ __align__(16) float js[];  // [cells][P], then the staged site pairs
+    constexpr uint32_t P = B * B;
+    const uint32_t qq = q * q, QI = joint_states(q, GI), QJ = joint_states(q, GJ);
+    const uint32_t s = blockIdx.x % g.nslices, chunk = blockIdx.x / g.nslices;
+    uint32_t bi, bj;
+    joint_coords<GI, GJ>(s, g.nbJ, bi, bj);
+    const uint32_t i0 = bi * (B * GI), j0 = bj * (B * GJ);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = T / 32;
+
+    if constexpr (GI * GJ == 1) {
+        // lane l stages cell c0 + l % 8 of pair p0 + l / 8 (global reads of 8
+        // consecutive cells of 4 pairs)
+        const uint32_t cgroups = (qq + 7) / 8;
+        for (uint32_t t = warp; t < cgroups * (P / 4); t += nwarps) {
+            const uint32_t c = (t % cgroups) * 8 + (lane & 7), p = (t / cgroups) * 4 + (lane >> 3);
+            const uint32_t i = i0 + p / B, j = j0 + p % B;
+            if (c < qq) js[c * P + p] = (i < j && j < L) ? __ldg(&J[pair_index(i, j, L) * qq + c]) : 0.0f;
         }
-        return;
+    } else {
+        float *raw = js + joint_table(q, B, GI, GJ);
+        const uint32_t S = joint_stage_pair(q, GJ), R = joint_stage_row(q, B, GJ);
+#pragma unroll 4
+        for (uint32_t t = warp; t < GI * B * GJ * B; t += nwarps) {
+            const uint32_t r = t / (GJ * B), cc = t % (GJ * B), i = i0 + r, j = j0 + cc;
+            const bool ok = i < j && j < L;
+            for (uint32_t e = lane; e < qq; e += 32) raw[r * R + cc * S + e] = ok ? __ldg(&J[pair_index(i, j, L) * qq + e]) : 0.0f;
+        }
+        __syncthreads();
+        // each cell: the sum of its site pairs' couplings, rounded once
+        for (uint32_t c = warp; c < QI * QJ; c += nwarps) {
+            const uint32_t A = c / QJ, Bc = c - A * QJ;
+            uint32_t a[GI], b[GJ];
+            a[0] = GI == 1 ? A : A % q;
+            if constexpr (GI == 2) a[1] = A / q;
+            b[0] = GJ == 1 ? Bc : Bc % q;
+            if constexpr (GJ == 2) b[1] = Bc / q;
+#pragma unroll
+            for (uint32_t p = lane; p < P; p += 32) {
+                const float *src = raw + (p / B) * GI * R + (p % B) * GJ * S;
+                double v = 0.0;
+#pragma unroll
+                for (int x = 0; x < GI; ++x)
+#pragma unroll
+                    for (int y = 0; y < GJ; ++y) v += (double)src[x * R + y * S + a[x] * q + b[y]];
+                js[c * P + p] = (float)v;
+            }
+        }
     }
-    // two sequences per thread: two independent chains of loads in flight
-    for (uint32_t n = nbeg + threadIdx.x; n < nend; n += 2 * blockDim.x) {
-        const uint32_t n2 = n + blockDim.x;
-        const bool two = n2 < nend;
-        uint32_t wI[B / 4], wJ[B / 4], vI[B / 4], vJ[B / 4];
-        load_block_words<B>(seq, buflen, n, bi, swords, wI);
-        load_block_words<B>(seq, buflen, n, bj, swords, wJ);
-        load_block_words<B>(seq, buflen, two ? n2 : n, bi, swords, vI);
-        load_block_words<B>(seq, buflen, two ? n2 : n, bj, swords, vJ);
-        uint32_t row[B], col[B];
-        lane_offsets<B>(wI, wJ, q, lane, row, col);
-        const double e1 = lane_energy<B>(jbase, row, col);
-        lane_offsets<B>(vI, vJ, q, lane, row, col);
-        const double e2 = lane_energy<B>(jbase, row, col);
-        atomicAdd(&acc[n], (unsigned long long)__double2ll_rn(e1 * FIX_SCALE));
-        if (two) atomicAdd(&acc[n2], (unsigned long long)__double2ll_rn(e2 * FIX_SCALE));
-    }
+    __syncthreads();
+
+    const uint32_t nbeg = chunk * g.chunk, nend = min(nseq, nbeg + g.chunk);
+    const uint32_t jbase = (uint32_t)__cvta_generic_to_shared(js);
+    joint_sequences<B, GI, GJ>(seq, buflen, nbeg, nend, L, q, bi, bj,
+                               [&](const uint32_t(&row)[B], const uint32_t(&col)[B], uint32_t n) {
+                                   const double e = lane_energy<B>(jbase, row, col);
+                                   atomicAdd(&acc[n], (unsigned long long)__double2ll_rn(e * FIX_SCALE));
+                               });
 }
 
 template <int B, bool CONS>
@@ -183,24 +217,6 @@ __global__ void __launch_bounds__(512, 2) k_energies(const float *__restrict__ J
     const int kind = slice_kind(bi, bj, j0, B, L);
     const uint32_t nbeg = chunk * g.chunk;
     const uint32_t nend = min(nseq, nbeg + g.chunk);
-
-    if constexpr (!CONS && B >= 8) {
-        if (kind == SLICE_FULL) {
-            // cell-major table [cell][P] for lanes over pairs: lane l
-            // stages cell c0 + l % 8 of pair p0 + l / 8 (global reads of 8
-            // consecutive cells of 4 pairs)
-            constexpr uint32_t P = B * B;
-            const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-            const uint32_t cgroups = (qq + 7) / 8;
-            for (uint32_t t = warp; t < cgroups * (P / 4); t += nwarps) {
-                const uint32_t c = (t % cgroups) * 8 + (lane & 7), p = (t / cgroups) * 4 + (lane >> 3);
-                if (c < qq) js[c * P + p] = __ldg(&J[pair_index(i0 + p / B, j0 + p % B, L) * qq + c]);
-            }
-            __syncthreads();
-            energies_chunk_lanes<B>(js, seq, buflen, nbeg, nend, acc, L, q, bi, bj);
-            return;
-        }
-    }
 
     // Stage the slice's couplings: for each i, pairs (i, jlo..jhi-1) are
     // contiguous in the packed table.
@@ -251,16 +267,35 @@ static int launch_energies(const float *J, const uint32_t *seq, uint32_t buflen,
     return check_launch("mi3_energies");
 }
 
+template <typename C>
+static int launch_energies_joint(const float *J, const uint32_t *seq, uint32_t buflen, uint32_t nseq,
+                                 unsigned long long *acc, uint32_t L, uint32_t q, cudaStream_t st) {
+    const JointGeom g = joint_geom<C>(L, nseq);
+    const size_t smem = joint_smem(q, C::B, C::GI, C::GJ);
+    auto kernel = k_energies_joint<C::B, C::GI, C::GJ, C::T>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const uint64_t nblk = (uint64_t)g.nslices * g.nchunks;
+    if (nblk > 0x7fffffffull) return fail(MI3_ERR_ARG, "mi3_energies: grid too large");
+    kernel<<<(uint32_t)nblk, C::T, smem, st>>>(J, seq, buflen, nseq, acc, L, q, g);
+    return check_launch("mi3_energies");
+}
+
 template <bool CONS>
 static int dispatch_energies(const float *J, const uint32_t *seq, uint32_t buflen, uint32_t nseq,
                              unsigned long long *acc, uint32_t L, uint32_t q, const uint8_t *cons,
                              cudaStream_t st) {
-    switch (pick_block(q, 116 * 1024, 16)) {
-        case 16: return launch_energies<16, CONS>(J, seq, buflen, nseq, acc, L, q, cons, st);
-        case 8: return launch_energies<8, CONS>(J, seq, buflen, nseq, acc, L, q, cons, st);
-        case 4: return launch_energies<4, CONS>(J, seq, buflen, nseq, acc, L, q, cons, st);
-        default: return fail(MI3_ERR_ARG, "mi3_energies: q too large");
+    if constexpr (!CONS) {
+        int rc = MI3_OK;
+        if (joint_dispatch(q, [&](auto cfg) { rc = launch_energies_joint<decltype(cfg)>(J, seq, buflen, nseq, acc, L, q, st); }))
+            return rc;
     }
+    const uint32_t B = pick_block(q, 116 * 1024, 16);
+    if constexpr (CONS) {
+        if (B == 16) return launch_energies<16, true>(J, seq, buflen, nseq, acc, L, q, cons, st);
+        if (B == 8) return launch_energies<8, true>(J, seq, buflen, nseq, acc, L, q, cons, st);
+    }
+    if (B == 4) return launch_energies<4, CONS>(J, seq, buflen, nseq, acc, L, q, cons, st);
+    return fail(MI3_ERR_ARG, "mi3_energies: q too large");
 }
 
 // ------------------------------------------------------- consensus gauge

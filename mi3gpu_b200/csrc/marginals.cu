@@ -9,7 +9,7 @@
 // increments them with shared-memory atomics for a chunk of sequences, and
 // flushes them once.  Counts are integers, so they are exact whatever the
 // order.
-#include "tiling.cuh"
+#include "joint.cuh"
 
 namespace mi3 {
 
@@ -121,60 +121,92 @@ __device__ __forceinline__ void hist_chunk(uint32_t *h, const uint32_t *__restri
     }
 }
 
-// Full slices with lanes over pairs (tiling.cuh): the histograms are
-// [cell][P] and each lane visits the pairs in its own rotated order, so the
-// 32 lanes of a shared-memory reduction always hit 32 different banks and
-// different bins (no serialised same-bin adds either).
-template <int B>
-__device__ __forceinline__ void lane_hist(uint32_t hbase, const uint32_t (&row)[B], const uint32_t (&col)[B],
-                                          uint32_t inc) {
-#pragma unroll
-    for (int tl = 0; tl < B; ++tl) {
-        const uint32_t c = hbase + col[tl];
-#pragma unroll
-        for (int th = 0; th < B; ++th)
-            asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(c + row[th]), "r"(inc));
-    }
-}
+// Histograms over joint sites (joint.cuh): [cell][P] bins, each lane adds to
+// the pairs in its own rotated order, so the 32 lanes of a shared-memory
+// reduction always hit 32 different banks and different bins (no serialised
+// same-bin adds either).  The flush splits a joint bin back into the site
+// pairs it counts; sums of a chunk's increments fit u32 (fixed_shift).  Bound by
+// instruction issue, two per (sequence, joint pair), and the shared-memory
+// reductions; figures in joint.cuh.
+template <int B, int GI, int GJ, int T, bool WEIGHTED>
+__global__ void __launch_bounds__(T, 1024 / T) k_pairhist_joint(const uint32_t *__restrict__ seq, uint32_t buflen,
+                                                               uint32_t nseq, const float *__restrict__ weights,
+                                                               const unsigned int *__restrict__ wmax_bits,
+                                                               uint32_t *out, uint32_t L, uint32_t q, JointGeom g,
+                                                               uint64_t nbins) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint32_t *h = reinterpret_cast<uint32_t *>(smem_raw);  // [cells][P], then the site pairs' bins
+    constexpr uint32_t P = B * B;
+    const uint32_t qq = q * q, QJ = joint_states(q, GJ), ncell = joint_states(q, GI) * QJ;
+    const uint32_t s = blockIdx.x % g.nslices, chunk = blockIdx.x / g.nslices;
+    uint32_t bi, bj;
+    joint_coords<GI, GJ>(s, g.nbJ, bi, bj);
+    const uint32_t i0 = bi * (B * GI), j0 = bj * (B * GJ);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = T / 32;
+    for (uint32_t k = threadIdx.x; k < ncell * P; k += T) h[k] = 0u;
+    float scale = 1.0f;
+    if constexpr (WEIGHTED) scale = ldexpf(1.0f, fixed_shift(__uint_as_float(*wmax_bits), g.chunk));
+    __syncthreads();
 
-template <int B, bool WEIGHTED>
-__device__ __forceinline__ void hist_chunk_lanes(uint32_t *h, const uint32_t *__restrict__ seq, uint32_t buflen,
-                                                 uint32_t nbeg, uint32_t nend, const float *__restrict__ weights,
-                                                 float scale, uint32_t L, uint32_t q, uint32_t bi, uint32_t bj) {
-    const uint32_t swords = (L - 1) / 4 + 1;
-    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t nbeg = chunk * g.chunk, nend = min(nseq, nbeg + g.chunk);
     const uint32_t hbase = (uint32_t)__cvta_generic_to_shared(h);
-    if constexpr (B == 16) {
-        for (uint32_t n = nbeg + threadIdx.x; n < nend; n += blockDim.x) {
-            uint32_t wI[B / 4], wJ[B / 4];
-            load_block_words<B>(seq, buflen, n, bi, swords, wI);
-            load_block_words<B>(seq, buflen, n, bj, swords, wJ);
-            uint32_t inc = 1u;
-            if constexpr (WEIGHTED) inc = __float2uint_rn(__ldg(&weights[n]) * scale);
-            uint32_t row[B], col[B];
-            lane_offsets<B>(wI, wJ, q, lane, row, col);
-            lane_hist<B>(hbase, row, col, inc);
-        }
-        return;
-    }
-    for (uint32_t n = nbeg + threadIdx.x; n < nend; n += 2 * blockDim.x) {
-        const uint32_t n2 = n + blockDim.x;
-        const bool two = n2 < nend;
-        uint32_t wI[B / 4], wJ[B / 4], vI[B / 4], vJ[B / 4];
-        load_block_words<B>(seq, buflen, n, bi, swords, wI);
-        load_block_words<B>(seq, buflen, n, bj, swords, wJ);
-        load_block_words<B>(seq, buflen, two ? n2 : n, bi, swords, vI);
-        load_block_words<B>(seq, buflen, two ? n2 : n, bj, swords, vJ);
-        uint32_t inc1 = 1u, inc2 = 1u;
+    joint_sequences<B, GI, GJ>(seq, buflen, nbeg, nend, L, q, bi, bj,
+                               [&](const uint32_t(&row)[B], const uint32_t(&col)[B], uint32_t n) {
+                                   uint32_t inc = 1u;
+                                   if constexpr (WEIGHTED) inc = __float2uint_rn(__ldg(&weights[n]) * scale);
+#pragma unroll
+                                   for (int tl = 0; tl < B; ++tl) {
+                                       const uint32_t c = hbase + col[tl];
+#pragma unroll
+                                       for (int th = 0; th < B; ++th)
+                                           asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(c + row[th]), "r"(inc));
+                                   }
+                               });
+    __syncthreads();
+
+    auto flush = [&](uint64_t dst, uint32_t v) {
         if constexpr (WEIGHTED) {
-            inc1 = __float2uint_rn(__ldg(&weights[n]) * scale);
-            inc2 = two ? __float2uint_rn(__ldg(&weights[n2]) * scale) : 0u;
+            // this chunk's partial sums: a plain store into its own plane
+            out[(uint64_t)chunk * nbins + dst] = v;
+        } else if (g.nchunks > 1) {
+            if (v) atomicAdd(out + dst, v);
+        } else {
+            out[dst] = v;
         }
-        uint32_t row[B], col[B];
-        lane_offsets<B>(wI, wJ, q, lane, row, col);
-        lane_hist<B>(hbase, row, col, inc1);
-        lane_offsets<B>(vI, vJ, q, lane, row, col);
-        lane_hist<B>(hbase, row, col, two ? inc2 : 0u);
+    };
+    if constexpr (GI * GJ == 1) {
+        // lane l takes cell c0 + l % 8 of pair p0 + l / 8 -- global writes of
+        // 8 consecutive cells of 4 pairs
+        const uint32_t cgroups = (qq + 7) / 8;
+        for (uint32_t t = warp; t < cgroups * (P / 4); t += nwarps) {
+            const uint32_t c = (t % cgroups) * 8 + (lane & 7), p = (t / cgroups) * 4 + (lane >> 3);
+            const uint32_t i = i0 + p / B, j = j0 + p % B;
+            if (c < qq && i < j && j < L) flush(pair_index(i, j, L) * qq + c, h[c * P + p]);
+        }
+    } else {
+        uint32_t *raw = h + joint_table(q, B, GI, GJ);
+        const uint32_t S = joint_stage_pair(q, GJ), R = joint_stage_row(q, B, GJ);
+        const uint32_t rowother = GI == 2 ? q : 1, colother = GJ == 2 ? q : 1;
+        // bin (a, b) of sub-pair (x, y): the joint bins over the other residues
+        for (uint32_t t = warp; t < GI * GJ * qq; t += nwarps) {
+            const uint32_t xy = t / qq, e = t - xy * qq, a = e / q, b = e - a * q;
+            const uint32_t x = xy / GJ, y = xy % GJ;
+            const uint32_t A0 = GI == 2 && x ? a * q : a, dA = GI == 2 && x ? 1 : q;
+            const uint32_t B0 = GJ == 2 && y ? b * q : b, dB = GJ == 2 && y ? 1 : q;
+#pragma unroll
+            for (uint32_t p = lane; p < P; p += 32) {
+                uint32_t v = 0;
+                for (uint32_t u = 0; u < rowother; ++u)
+                    for (uint32_t w = 0; w < colother; ++w) v += h[((A0 + u * dA) * QJ + B0 + w * dB) * P + p];
+                raw[((p / B) * GI + x) * R + ((p % B) * GJ + y) * S + e] = v;
+            }
+        }
+        __syncthreads();
+        for (uint32_t t = warp; t < GI * B * GJ * B; t += nwarps) {
+            const uint32_t r = t / (GJ * B), cc = t % (GJ * B), i = i0 + r, j = j0 + cc;
+            if (!(i < j && j < L)) continue;
+            for (uint32_t e = lane; e < qq; e += 32) flush(pair_index(i, j, L) * qq + e, raw[r * R + cc * S + e]);
+        }
     }
 }
 
@@ -206,31 +238,6 @@ __global__ void __launch_bounds__(512, 2) k_pairhist(const uint32_t *__restrict_
     const uint32_t nbeg = chunk * g.chunk;
     const uint32_t nend = min(nseq, nbeg + g.chunk);
     const int kind = slice_kind(bi, bj, j0, B, L);
-    if constexpr (!CONS && B >= 8) {
-        if (kind == SLICE_FULL) {
-            hist_chunk_lanes<B, WEIGHTED>(h, seq, buflen, nbeg, nend, weights, scale, L, q, bi, bj);
-            __syncthreads();
-            // flush the [cell][P] table: lane l takes cell c0 + l % 8 of pair
-            // p0 + l / 8 -- global writes of 8 consecutive cells of 4 pairs
-            constexpr uint32_t P = B * B;
-            const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-            const uint32_t cgroups = (qq + 7) / 8;
-            for (uint32_t t = warp; t < cgroups * (P / 4); t += nwarps) {
-                const uint32_t c = (t % cgroups) * 8 + (lane & 7), p = (t / cgroups) * 4 + (lane >> 3);
-                if (c >= qq) continue;
-                const uint32_t v = h[c * P + p];
-                const uint64_t dst = pair_index(i0 + p / B, j0 + p % B, L) * qq + c;
-                if constexpr (WEIGHTED) {
-                    reinterpret_cast<uint32_t *>(out)[(uint64_t)chunk * nbins + dst] = v;
-                } else if (g.nchunks > 1) {
-                    if (v) atomicAdd(reinterpret_cast<uint32_t *>(out) + dst, v);
-                } else {
-                    reinterpret_cast<uint32_t *>(out)[dst] = v;
-                }
-            }
-            return;
-        }
-    }
     switch (kind) {
         case SLICE_FULL:
             hist_chunk<B, SLICE_FULL, WEIGHTED, CONS>(h, seq, buflen, nbeg, nend, weights, scale, L, q, bi, bj,
@@ -293,17 +300,54 @@ __global__ void k_chunks_to_float(const uint32_t *__restrict__ part, uint32_t nc
 
 constexpr uint32_t WMARG_CHUNK = 65536;  // sequences per CTA (fixed-point headroom)
 
-// The weighted chunk also sets the fixed-point scale (fixed_shift), so it is
-// never longer than what about 8 CTAs per SM would give, nor than
-// WMARG_CHUNK; each chunk costs a plane of bins, written and read once (the
-// larger overhead).
+// Chunks of a weighted pass.  The chunk length also sets the fixed-point
+// scale (fixed_shift), so a pass is cut into at least the chunks that about 8
+// CTAs per SM of the pair-major tiling would take, and no chunk is longer than
+// WMARG_CHUNK.  Each chunk costs a plane of bins, written and read once
+// (counted as 4096 sequences), against whole waves of CTAs.  The number never
+// falls as nseq grows (the plane term's weight falls), so a workspace for nseq
+// sequences also serves fewer.
+static uint32_t wmarg_split(uint32_t L, uint32_t q, uint32_t nseq) {
+    const uint32_t B = pick_block(q, 116 * 1024, 16);
+    if (!B) return 1;
+    const uint32_t nb = (L + B - 1) / B, pair_slices = nb * (nb + 1) / 2;
+    const uint32_t least = (148 * 8 + pair_slices - 1) / pair_slices;
+    uint32_t ns = pair_slices, resident = PAIR_RESIDENT;
+    joint_dispatch(q, [&](auto cfg) {
+        using C = decltype(cfg);
+        JointGeom g;
+        joint_slices(L, C::B, C::GI, C::GJ, &g);
+        ns = g.nslices;
+        resident = 148 * (1024 / C::T);
+    });
+    const uint32_t w0 = (least * ns + resident - 1) / resident;
+    uint32_t best_k = least;
+    double best = 1e30;
+    for (uint32_t w = w0; w < w0 + 24; ++w) {
+        const uint32_t k = std::max(least, (uint32_t)((uint64_t)w * resident / ns));
+        const double cost = (double)w / k * (1.0 + k * 4096.0 / nseq);
+        if (cost < best) {
+            best = cost;
+            best_k = k;
+        }
+    }
+    return best_k;
+}
+
+uint32_t wmarg_fixed_chunk(uint32_t L, uint32_t q, uint32_t nseq) {
+    if (!nseq) return WMARG_CHUNK;
+    const uint32_t chunk = ((nseq - 1) / wmarg_split(L, q, nseq) + 1 + 255) & ~255u;
+    return std::min(std::max(chunk, PAIR_MIN_CHUNK), WMARG_CHUNK);
+}
+
 template <int B, bool WEIGHTED>
-static SliceGeom pairhist_geom(uint32_t L, uint32_t nseq) {
-    if (!WEIGHTED) return make_geom(L, B, nseq);
-    const uint32_t nb = (L + B - 1) / B, nslices = nb * (nb + 1) / 2;
-    const uint32_t want = (148 * 8 + nslices - 1) / nslices;
-    const uint32_t longest = (std::max<uint32_t>((nseq + want - 1) / want, 2048) + 255) & ~255u;
-    return make_geom(L, B, nseq, std::min(longest, WMARG_CHUNK), 2 * PAIR_CTA_OVERHEAD);
+static SliceGeom pairhist_geom(uint32_t L, uint32_t q, uint32_t nseq) {
+    SliceGeom g = make_geom(L, B, nseq);
+    if (WEIGHTED) {
+        g.chunk = wmarg_fixed_chunk(L, q, nseq);
+        g.nchunks = (nseq - 1) / g.chunk + 1;
+    }
+    return g;
 }
 
 // Per-site residue sums over blocks of at most per_cta sequences (<= the pair
@@ -467,11 +511,50 @@ inline bool cons_supported(uint32_t L, uint32_t q) {
     return q <= 64 && ((size_t)L * q * 4 + L) <= 160 * 1024;
 }
 
+// The weighted pass after its histogram kernel: planes -> float.
+static int finish_wmarg(const WmargWs &W, uint32_t nchunks, uint32_t chunk, void *out, uint64_t nbins, cudaStream_t st) {
+    int rc = check_launch("mi3_weighted_marg");
+    if (rc) return rc;
+    k_chunks_to_float<<<(uint32_t)((nbins + 255) / 256), 256, 0, st>>>(W.planes, nchunks, W.wmax, chunk,
+                                                                      reinterpret_cast<float *>(out), nbins);
+    return check_launch("mi3_weighted_marg: planes");
+}
+
+template <typename C, bool WEIGHTED>
+static int launch_pairhist_joint(const uint32_t *seq, uint32_t buflen, uint32_t nseq, const float *w,
+                                 unsigned char *ws, void *out, uint32_t L, uint32_t q, cudaStream_t st) {
+    JointGeom g = joint_geom<C>(L, nseq);
+    if (WEIGHTED) {
+        g.chunk = wmarg_fixed_chunk(L, q, nseq);
+        g.nchunks = (nseq - 1) / g.chunk + 1;
+    }
+    const size_t smem = joint_smem(q, C::B, C::GI, C::GJ);
+    auto kernel = k_pairhist_joint<C::B, C::GI, C::GJ, C::T, WEIGHTED>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const uint64_t nblk = (uint64_t)g.nslices * g.nchunks;
+    if (nblk > 0x7fffffffull) return fail(MI3_ERR_ARG, "pair histogram: grid too large");
+    const uint64_t nbins = npairs_of(L) * q * q;
+    if (!WEIGHTED) {
+        if (g.nchunks > 1 && cudaMemsetAsync(out, 0, nbins * 4, st) != cudaSuccess)
+            return check_launch("bicounts: memset");
+        kernel<<<(uint32_t)nblk, C::T, smem, st>>>(seq, buflen, nseq, w, nullptr, reinterpret_cast<uint32_t *>(out), L,
+                                                   q, g, nbins);
+        return check_launch("mi3_bicounts");
+    }
+    // every bin of every chunk plane is stored by the kernel: only the
+    // scalars need clearing
+    WmargWs W = wmarg_ws(ws, L, q);
+    if (cudaMemsetAsync(ws, 0, 256, st) != cudaSuccess) return check_launch("weighted marg: memset");
+    k_wmax<<<296, 512, 0, st>>>(w, nseq, W.wmax);
+    kernel<<<(uint32_t)nblk, C::T, smem, st>>>(seq, buflen, nseq, w, W.wmax, W.planes, L, q, g, nbins);
+    return finish_wmarg(W, g.nchunks, g.chunk, out, nbins, st);
+}
+
 template <int B, bool WEIGHTED, bool CONS>
 static int launch_pairhist(const uint32_t *seq, uint32_t buflen, uint32_t nseq, const float *w,
                            unsigned char *ws, void *out, uint32_t L, uint32_t q, const uint8_t *cons,
                            cudaStream_t st) {
-    SliceGeom g = pairhist_geom<B, WEIGHTED>(L, nseq);
+    SliceGeom g = pairhist_geom<B, WEIGHTED>(L, q, nseq);
     size_t smem = (size_t)B * B * q * q * 4;
     cudaFuncSetAttribute(k_pairhist<B, WEIGHTED, CONS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     uint64_t nblk = (uint64_t)g.nslices * g.nchunks;
@@ -492,13 +575,9 @@ static int launch_pairhist(const uint32_t *seq, uint32_t buflen, uint32_t nseq, 
     k_wmax<<<296, 512, 0, st>>>(w, nseq, W.wmax);
     k_pairhist<B, true, CONS><<<(uint32_t)nblk, 512, smem, st>>>(seq, buflen, nseq, w, W.wmax, W.planes, L, q, g,
                                                                 nbins, cons);
+    if (!CONS) return finish_wmarg(W, g.nchunks, g.chunk, out, nbins, st);
     int rc = check_launch("mi3_weighted_marg");
     if (rc) return rc;
-    if (!CONS) {
-        k_chunks_to_float<<<(uint32_t)((nbins + 255) / 256), 256, 0, st>>>(W.planes, g.nchunks, W.wmax, g.chunk,
-                                                                          reinterpret_cast<float *>(out), nbins);
-        return check_launch("mi3_weighted_marg: planes");
-    }
     const uint32_t per_cta = std::min<uint32_t>(g.chunk, std::max<uint32_t>(256, (nseq + 148 * 4 - 1) / (148 * 4)));
     const size_t ssm = (size_t)L * q * 4 + L;
     if (ssm > 48 * 1024)
@@ -527,12 +606,13 @@ static int dispatch_pairhist(const uint32_t *seq, uint32_t buflen, uint32_t nseq
             }
         }
     }
-    switch (B) {
-        case 16: return launch_pairhist<16, WEIGHTED, false>(seq, buflen, nseq, w, ws, out, L, q, nullptr, st);
-        case 8: return launch_pairhist<8, WEIGHTED, false>(seq, buflen, nseq, w, ws, out, L, q, nullptr, st);
-        case 4: return launch_pairhist<4, WEIGHTED, false>(seq, buflen, nseq, w, ws, out, L, q, nullptr, st);
-        default: return fail(MI3_ERR_ARG, "pair histogram: q too large");
-    }
+    int rc = MI3_OK;
+    if (joint_dispatch(q, [&](auto cfg) {
+            rc = launch_pairhist_joint<decltype(cfg), WEIGHTED>(seq, buflen, nseq, w, ws, out, L, q, st);
+        }))
+        return rc;
+    if (B == 4) return launch_pairhist<4, WEIGHTED, false>(seq, buflen, nseq, w, ws, out, L, q, nullptr, st);
+    return fail(MI3_ERR_ARG, "pair histogram: q too large");
 }
 
 __global__ void k_bicounts_to_bimarg(const uint32_t *__restrict__ c, float *bi, float nseq, uint64_t n) {
@@ -598,26 +678,11 @@ extern "C" int mi3_bicounts(const uint32_t *seqmem, uint32_t buflen, uint32_t ns
                                     as_stream(stream));
 }
 
-namespace mi3 {
-uint32_t wmarg_fixed_chunk(uint32_t L, uint32_t q, uint32_t nseq) {
-    switch (pick_block(q, 116 * 1024, 16)) {
-        case 16: return pairhist_geom<16, true>(L, nseq).chunk;
-        case 8: return pairhist_geom<8, true>(L, nseq).chunk;
-        case 4: return pairhist_geom<4, true>(L, nseq).chunk;
-        default: return WMARG_CHUNK;
-    }
-}
-}  // namespace mi3
-
 extern "C" size_t mi3_weighted_marg_workspace(uint32_t L, uint32_t q, uint32_t nseq) {
-    uint32_t nchunks = 1;
-    switch (pick_block(q, 116 * 1024, 16)) {
-        case 16: nchunks = pairhist_geom<16, true>(L, nseq).nchunks; break;
-        case 8: nchunks = pairhist_geom<8, true>(L, nseq).nchunks; break;
-        case 4: nchunks = pairhist_geom<4, true>(L, nseq).nchunks; break;
-        default: break;
-    }
-    return 256 + usite_bytes(L, q) + (size_t)std::max<uint32_t>(nchunks, 1) * npairs_of(L) * q * q * 4;
+    // at least the chunks of any call with up to nseq sequences
+    const uint32_t split = nseq ? std::min(wmarg_split(L, q, nseq), nseq / PAIR_MIN_CHUNK + 1) : 1;
+    const uint32_t nchunks = std::max(nseq / WMARG_CHUNK + 1, split);
+    return 256 + usite_bytes(L, q) + (size_t)nchunks * npairs_of(L) * q * q * 4;
 }
 
 extern "C" int mi3_weighted_marg(const float *weights, const uint32_t *seqmem, uint32_t buflen,

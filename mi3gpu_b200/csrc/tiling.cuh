@@ -58,29 +58,35 @@ inline uint32_t pick_block(uint32_t q, size_t budget, uint32_t max_b = 32) {
 // even out.
 constexpr uint32_t PAIR_RESIDENT = 148 * 2, PAIR_CTA_OVERHEAD = 2048, PAIR_MIN_CHUNK = 1024, PAIR_MIN_WAVES = 3;
 
+inline uint32_t pick_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident, uint32_t max_chunk,
+                           uint32_t overhead) {
+    const uint32_t min_chunk = std::min(PAIR_MIN_CHUNK, max_chunk);
+    const uint32_t least = (nseq - 1) / max_chunk + 1;  // chunks that max_chunk asks for
+    const uint32_t most = std::max(least, (nseq - 1) / min_chunk + 1);
+    auto chunk_of = [&](uint32_t nc) { return std::min(max_chunk, ((nseq - 1) / nc + 1 + 255) & ~255u); };
+    uint32_t pick = chunk_of(least);
+    uint64_t best = ~0ull;
+    const uint32_t w0 = (uint32_t)(((uint64_t)nslices * least + resident - 1) / resident);
+    for (uint32_t w = std::max(w0, PAIR_MIN_WAVES); w < w0 + 24; ++w) {
+        const uint64_t fit = (uint64_t)w * resident / nslices;
+        const uint32_t chunk = chunk_of((uint32_t)std::min<uint64_t>(std::max<uint64_t>(fit, least), most));
+        const uint64_t cost = w * ((uint64_t)chunk + overhead);
+        if (cost < best) {
+            best = cost;
+            pick = chunk;
+        }
+        if (fit >= most) break;
+    }
+    return pick;
+}
+
 inline SliceGeom make_geom(uint32_t L, uint32_t B, uint32_t nseq, uint32_t max_chunk = 0xffffff00u,
                            uint32_t overhead = PAIR_CTA_OVERHEAD) {
     SliceGeom g;
     g.B = B;
     g.nb = (L + B - 1) / B;
     g.nslices = g.nb * (g.nb + 1) / 2;
-    const uint32_t min_chunk = std::min(PAIR_MIN_CHUNK, max_chunk);
-    const uint32_t least = (nseq - 1) / max_chunk + 1;  // chunks that max_chunk asks for
-    const uint32_t most = std::max(least, (nseq - 1) / min_chunk + 1);
-    auto chunk_of = [&](uint32_t nc) { return std::min(max_chunk, ((nseq - 1) / nc + 1 + 255) & ~255u); };
-    g.chunk = chunk_of(least);
-    uint64_t best = ~0ull;
-    const uint32_t w0 = (uint32_t)(((uint64_t)g.nslices * least + PAIR_RESIDENT - 1) / PAIR_RESIDENT);
-    for (uint32_t w = std::max(w0, PAIR_MIN_WAVES); w < w0 + 24; ++w) {
-        const uint64_t fit = (uint64_t)w * PAIR_RESIDENT / g.nslices;
-        const uint32_t chunk = chunk_of((uint32_t)std::min<uint64_t>(std::max<uint64_t>(fit, least), most));
-        const uint64_t cost = w * ((uint64_t)chunk + overhead);
-        if (cost < best) {
-            best = cost;
-            g.chunk = chunk;
-        }
-        if (fit >= most) break;
-    }
+    g.chunk = pick_chunk(g.nslices, nseq, PAIR_RESIDENT, max_chunk, overhead);
     g.nchunks = (nseq - 1) / g.chunk + 1;
     return g;
 }
@@ -154,12 +160,12 @@ __device__ __forceinline__ uint32_t slice_row(const uint32_t (&wI)[B / 4], int i
     return (uint32_t)ii * B * qq + block_byte<B>(wI, ii, q - 1) * q;
 }
 
-// ------------------------------------------------ lanes over pairs (full slices)
+// ------------------------------------------------ lanes over pairs
 // In a slice table laid out pair-major, [p][cell], the 32 sequences of a warp
 // all visit pair p at the same time and gather 32 random cells: about 3.3
-// shared-memory wavefronts per warp instruction.  For full slices (every
-// pair valid) the pair kernels can instead lay the table out cell-major,
-// [cell][p] with P = B*B pairs (p = ii*B + jj).  Lane w = B*wh + wl visits, at
+// shared-memory wavefronts per warp instruction.  For q <= 21 (joint.cuh) the
+// pair kernels lay the table out cell-major instead, [cell][p] with P = B*B
+// pairs (p = ii*B + jj).  Lane w = B*wh + wl visits, at
 // step (th, tl), the pair ii = (th + wh) mod B, jj = (tl + wl) mod B.  Its bank
 // is (ii*B + jj) mod 32: the B lanes of one wh hold B different jj, and the
 // 32/B values of wh hold ii that differ mod 32/B, so the 32 lanes use 32
@@ -187,26 +193,6 @@ __device__ __forceinline__ void rotate_block(const uint32_t (&w)[B / 4], uint32_
     }
 #pragma unroll
     for (int k = 0; k < W; ++k) o[k] = __funnelshift_r(t[k], t[(k + 1) % W], rb);
-}
-
-// Byte offsets, in a [cell][P] float table, of lane's row (site ii of block
-// I with residue a: a*q*P + ii*B) and column (site jj of block J with
-// residue b: b*P + jj) terms, in rotated order.
-template <int B>
-__device__ __forceinline__ void lane_offsets(const uint32_t (&wI)[B / 4], const uint32_t (&wJ)[B / 4], uint32_t q,
-                                             uint32_t lane, uint32_t (&row)[B], uint32_t (&col)[B]) {
-    constexpr uint32_t P = B * B;
-    const uint32_t wh = lane / B, wl = lane % B;
-    uint32_t rI[B / 4], rJ[B / 4];
-    rotate_block<B>(wI, wh, rI);
-    rotate_block<B>(wJ, wl, rJ);
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-        const uint32_t a = min((rI[k >> 2] >> (8 * (k & 3))) & 0xffu, q - 1);
-        const uint32_t b = min((rJ[k >> 2] >> (8 * (k & 3))) & 0xffu, q - 1);
-        row[k] = 4 * (a * q * P + ((k + wh) & (B - 1)) * B);
-        col[k] = 4 * (b * P + ((k + wl) & (B - 1)));
-    }
 }
 
 // ---------------------------------------------------------------- consensus
