@@ -40,6 +40,10 @@ METRIC = "site-updates/s"
 
 # (kernel, L, q) -> what bounds the kernel, from its ncu capture (cited)
 BINDING_CITED = {
+    ("k_metropolis_rot", 232, 21): {
+        "resource": "instruction issue and the shared-memory pipe together", "issue_active": 0.748,
+        "l1tex_throughput": 0.601, "shared_wavefronts_per_update": 14.6,
+        "source": "ncu sections (profiles/metropolis_rot_L232_q21.md)"},
     ("k_metropolis_skew", 232, 21): {
         "resource": "instruction issue", "issue_active": 0.768, "l1tex_throughput": 0.476,
         "shared_wavefronts_per_update": 18.4, "source": "ncu --set full (profiles/metropolis_skew_L232_q21.md)"},
@@ -183,7 +187,8 @@ def run_gpu(args):
         from mi3gpu_b200.autotune import Autotuner
         t0 = time.time()
         tuned = Autotuner(ROOT / "_build" / "autotune.json").tune(gpu)
-        tuned = {"metropolis_plan": list(tuned["metropolis_plan"]), "count_kernel": tuned["count_kernel"],
+        tuned = {"metropolis_plan": list(tuned["metropolis_plan"]), "metropolis_rot": tuned["metropolis_rot"],
+                 "count_kernel": tuned["count_kernel"],
                  "tuning_s": round(time.time() - t0, 1)}
 
     s = gpu.stream
@@ -259,8 +264,9 @@ def run_gpu(args):
         peaks = json.loads(pk.read_text())
     hbm_peak = peaks.get("hbm_gbs", 6650.0)
     achieved = upd_launch * hbm_bytes_per_update / (per_launch_ms / 1e3) / 1e9
-    plan = gpu.sampler_plan()
-    kernel = "k_metropolis_skew" if plan[0] == "skew" else "k_metropolis"
+    rotated = gpu.sampler_kernel() == "rot"
+    plan = ("rot",) if rotated else gpu.sampler_plan()
+    kernel = "k_metropolis_rot" if rotated else "k_metropolis_skew" if plan[0] == "skew" else "k_metropolis"
     # DRAM bytes of one full-size launch (2^20 walkers x 2048 proposals),
     # measured by a one-pass ncu capture of this command's own launch; a
     # cited figure, not measured in this run

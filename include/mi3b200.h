@@ -142,6 +142,32 @@ int mi3_metropolis_skew(const float *Jtiles, uint32_t *rngstates, uint32_t posit
                         uint32_t *seqmem, uint32_t nseqs, uint32_t L, uint32_t q, uint32_t walkers_per_cta,
                         uint32_t replicas, int32_t *status, void *stream);
 
+/* Floats (4-byte words) of the coupling tables of mi3_metropolis_rot: L rows of
+ * chunks of [cells][32 columns], an error bound per (site, residue) and a copy
+ * of J.  0 outside 2 <= L <= 576, 2 <= q <= 21. */
+uint64_t mi3_jrot_floats(uint32_t L, uint32_t q);
+
+/* unpackfV (mcmc.cl:42-65) as launched by MCMCGPU.unpackJ
+ * (mcmcGPU.py:393-408), into those tables.  Jrot: mi3_jrot_floats(L, q)
+ * floats, 16-byte aligned. */
+int mi3_unpack_j_rot(const float *J, float *Jrot, uint32_t L, uint32_t q, void *stream);
+
+/* metropolis + DeltaEnergy (mcmc.cl:360-458) as launched by MCMCGPU.runMCMC
+ * (mcmcGPU.py:460-482), a third kernel design with identical results to
+ * mi3_metropolis (same walkers and RNG states, bit for bit): each warp sums
+ * the energy differences as integers in an order without bank conflicts, two
+ * sites to a gather for q <= 8, decides by a proven bound on the distance to
+ * the reference's float sum, and adds up in site order where the bound leaves
+ * the verdict open.  nseqs a multiple of 32.  lanes_per_walker: 1, 2 or 4 lanes
+ * share a walker's sites; walkers_per_cta: a multiple of 32 / lanes_per_walker
+ * with at most 512 to 1024 lanes per CTA, by L; 0 = by shape and nseqs, for
+ * either.  Residues >= q in seqmem are clamped to q - 1.  status: as
+ * mi3_metropolis. */
+int mi3_metropolis_rot(const float *Jrot, uint32_t *rngstates, uint32_t position_offset,
+                       const uint32_t *position_list, uint32_t nsteps, const float *betas, float beta,
+                       uint32_t *seqmem, uint32_t nseqs, uint32_t L, uint32_t q, uint32_t walkers_per_cta,
+                       uint32_t lanes_per_walker, int32_t *status, void *stream);
+
 /* gen_indep (mcmc.cl:170-244) as launched by MCMCGPU.gen_indep
  * (mcmcGPU.py:380-390); cprob is (L, q-1) cumulative probabilities
  * (MCMCGPU.prepare_indep, mcmcGPU.py:375-378). */

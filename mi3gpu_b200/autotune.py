@@ -1,9 +1,9 @@
 """Autotuner for the shape-dependent choices of the B200 kernels.
 
-The sampler's plan (the skewed-lane kernel with 512 or 768 walkers per CTA,
-or a tile plan of the row-streaming kernel: walkers per CTA, sites per
-streamed coupling chunk, ring stages, which `mi3_metropolis_plans` lists;
-all give the same trajectories), the bimarginal
+The sampler (the rotated kernel, or a plan: the skewed-lane kernel with 512 or
+768 walkers per CTA, or a tile plan of the row-streaming kernel: walkers per
+CTA, sites per streamed coupling chunk, ring stages, which
+`mi3_metropolis_plans` lists; all give the same trajectories), the bimarginal
 count kernel and the weighted-bimarginal kernel (shared-memory histogram or
 tcgen05 one-hot GEMM, which give the same integers) are picked per
 (L, q, walkers) by timing every candidate once on the device, from the caller's own walker state copied to scratch buffers
@@ -80,10 +80,10 @@ class Autotuner:
         os.replace(tmp, self.cache_path)
 
     def sampler_plan(self, gpu, probe_steps=None, reps=2):
-        """Fastest sampler plan for gpu's shape; times `reps` launches of
-        probe_steps proposals per walker (default two sweeps) for every plan
-        on scratch copies of the walkers and RNG states.  Returns
-        (plan, {plan: ms})."""
+        """Fastest plan of the skewed-lane and row-streaming kernels for gpu's
+        shape; times `reps` launches of probe_steps proposals per walker
+        (default two sweeps) for every plan on scratch copies of the walkers
+        and RNG states.  Returns (plan, {plan: ms})."""
         key = self._key("metropolis", gpu)
         if key in self.table:
             return _plan_from_json(self.table[key]["plan"]), self.table[key].get("ms", {})
@@ -91,7 +91,32 @@ class Autotuner:
         gpu.unpackJ(kind='rows')
         if gpu.skew_supported():
             gpu.unpackJ(kind='tiles')
-        L, q, N = gpu.L, gpu.q, gpu.nseq['main']
+        times, steps = self._time_sampler(gpu, sampler_plans(gpu.L, gpu.q, gpu.nseq['main']), probe_steps, reps)
+        best = min(times, key=times.get)
+        self.table[key] = {"plan": list(best), "ms": {_plan_key(k): v for k, v in times.items()},
+                           "probe_steps": steps}
+        self._save()
+        return best, self.table[key]["ms"]
+
+    def sampler_rot(self, gpu, probe_steps=None, reps=2):
+        """Whether the rotated sampler beats the best plan of sampler_plan for
+        gpu's shape, timed the same way."""
+        if not gpu.rot_supported():
+            return False
+        plan, ms = self.sampler_plan(gpu, probe_steps, reps)
+        key = self._key("metropolis_rot", gpu)
+        if key not in self.table:
+            gpu.require('MCMC')
+            gpu.unpackJ(kind='rot')
+            times, _ = self._time_sampler(gpu, [('rot',)], probe_steps, reps)
+            best = ms.get(_plan_key(plan))
+            self.table[key] = {"ms": times[('rot',)], "use": best is None or times[('rot',)] <= best}
+            self._save()
+        return bool(self.table[key]["use"])
+
+    @staticmethod
+    def _time_sampler(gpu, plans, probe_steps, reps):
+        L, q = gpu.L, gpu.q
         steps = int(probe_steps or min(gpu.nsteps, 2 * L))
         with torch.cuda.stream(gpu.stream):
             seq = gpu.bufs['seq main'].clone()
@@ -102,7 +127,7 @@ class Autotuner:
             pos = torch.randint(0, L, (steps,), generator=gen, dtype=torch.int32).to(gpu.device)
         s = gpu.stream.cuda_stream
         times = {}
-        for plan in sampler_plans(L, q, N):
+        for plan in plans:
             def run(plan=plan):
                 gpu.sampler_call(0, pos.data_ptr(), steps, seq.data_ptr(), rng.data_ptr(), status.data_ptr(), s,
                                  plan=plan)
@@ -110,11 +135,7 @@ class Autotuner:
             times[plan] = _events_time(gpu.stream, run, reps)
         if int(status.item()) != 0:
             raise RuntimeError("sampler reported status {} while tuning".format(int(status.item())))
-        best = min(times, key=times.get)
-        self.table[key] = {"plan": list(best), "ms": {_plan_key(k): v for k, v in times.items()},
-                           "probe_steps": steps}
-        self._save()
-        return best, self.table[key]["ms"]
+        return times, steps
 
     def count_kernel(self, gpu, reps=3):
         """'tc' or 'smem': the faster exact count kernel for gpu's shape
@@ -170,7 +191,8 @@ class Autotuner:
         """Tune every choice for gpu and install them on it."""
         plan, _ = self.sampler_plan(gpu)
         gpu.metro_plan = tuple(plan)
+        gpu.sampler_rot = self.sampler_rot(gpu)
         gpu.count_kernel = self.count_kernel(gpu)
         gpu.wmarg_kernel = self.wmarg_kernel(gpu)
-        return {"metropolis_plan": gpu.metro_plan, "count_kernel": gpu.count_kernel,
+        return {"metropolis_plan": gpu.metro_plan, "metropolis_rot": gpu.sampler_rot, "count_kernel": gpu.count_kernel,
                 "wmarg_kernel": gpu.wmarg_kernel}

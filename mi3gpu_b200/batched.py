@@ -310,6 +310,7 @@ class BatchedRounds:
     def _build(self, key, sweeps):
         for pr in self.problems:
             # workspaces are created before capture (no allocation inside it)
+            pr.gpu.ensure_sampler_tables()
             self._ws(pr.gpu, 'ws gauge', 'mi3_gauge_workspace', pr.L, pr.q)
             self._ws(pr.gpu, 'ws stats', 'mi3_bimarg_stats_workspace', pr.L)
             if 4 <= pr.q <= 32:

@@ -375,9 +375,10 @@ class MCMCGPU:
         return self.logevt('gen_indep', s)
 
     # ------------------------------------------------------------ couplings
-    # Two unpacked layouts exist: the padded rows ('Junpacked') of the
-    # row-streaming sampler and the chunk tiles ('Jtiles') of the skewed-lane
-    # sampler; both are rebuilt lazily after J changes.
+    # Three unpacked layouts exist: the padded rows ('Junpacked') of the
+    # row-streaming sampler, the chunk tiles ('Jtiles') of the skewed-lane
+    # sampler and the tables ('Jrot') of the rotated sampler; each is rebuilt
+    # lazily after J changes, when its sampler runs.
     @property
     def unpackedJ(self):
         return self._unpacked_rows
@@ -386,11 +387,23 @@ class MCMCGPU:
     def unpackedJ(self, v):
         self._unpacked_rows = v
         if not v:
-            self._unpacked_tiles = False
+            self._unpacked_tiles = self._unpacked_rot = False
+
+    def _sampler_layout(self):
+        if self.sampler_kernel() == 'rot':
+            return 'rot'
+        return 'tiles' if self.sampler_plan()[0] == 'skew' else 'rows'
 
     def unpackJ(self, wait_for=None, kind=None):
-        kind = kind or ('tiles' if self.sampler_plan()[0] == 'skew' else 'rows')
-        if kind == 'rows':
+        kind = kind or self._sampler_layout()
+        if kind == 'rot':
+            if self._unpacked_rot:
+                return wait_for
+            self._ensure_rot()
+            s = self._begin()
+            _lib.call('mi3_unpack_j_rot', self._ptr('J'), self._ptr('Jrot'), self.L, self.q, self._s)
+            self._unpacked_rot = True
+        elif kind == 'rows':
             if self._unpacked_rows:
                 return wait_for
             s = self._begin()
@@ -412,17 +425,37 @@ class MCMCGPU:
                 self.bufs['Jtiles'] = torch.empty(n * self.skew_replicas, dtype=torch.float32, device=self.device)
             self._unpacked_tiles = False
 
+    def _ensure_rot(self):
+        if 'Jrot' not in self.bufs:
+            n = int(_lib.query('mi3_jrot_floats', self.L, self.q))
+            with torch.cuda.device(self.device):
+                self.bufs['Jrot'] = torch.empty(n, dtype=torch.float32, device=self.device)
+            self._unpacked_rot = False
+
     def _unpack_tiles(self, stream_ptr):
         n = int(_lib.query('mi3_jtiles_floats', self.L, self.q))
         for r in range(self.skew_replicas):
             _lib.call('mi3_unpack_j_tiles', self._ptr('J'), self._ptr('Jtiles') + 4 * n * r, self.L, self.q,
                       stream_ptr)
 
+    def ensure_sampler_tables(self):
+        """Allocate the coupling tables of the sampler runMCMC runs (before a
+        stream capture, inside which nothing should be allocated)."""
+        layout = self._sampler_layout()
+        if layout == 'rot':
+            self._ensure_rot()
+        elif layout == 'tiles':
+            self._ensure_tiles()
+
     def unpack_call(self, stream_ptr):
-        """Launch the unpacking kernel of the current sampler plan on
+        """Launch the unpacking kernel of the sampler sampler_call runs on
         stream_ptr (for callers that record it themselves, e.g. in a CUDA
         graph, where J changes on the device)."""
-        if self.sampler_plan()[0] == 'skew':
+        layout = self._sampler_layout()
+        if layout == 'rot':
+            self._ensure_rot()
+            _lib.call('mi3_unpack_j_rot', self._ptr('J'), self._ptr('Jrot'), self.L, self.q, stream_ptr)
+        elif layout == 'tiles':
             self._ensure_tiles()
             self._unpack_tiles(stream_ptr)
         else:
@@ -446,8 +479,28 @@ class MCMCGPU:
         (L + 31 <= 288 with 512 or 768 walkers per CTA, else 256)."""
         return 2 <= self.q <= 21 and self.L + 31 <= 576 and self.nseq['main'] % 32 == 0
 
+    # The rotated sampler (mi3_metropolis_rot) gives the same trajectories and
+    # is the fastest where it applies (B200, site-updates/s against the best
+    # of the other two: L=93 q=4 2^18 6.0e10 / 2.4e10, L=232 q=21 2^20 1.16e10
+    # / 8.7e9, L=512 q=21 2^18 3.5e9 / 3.2e9).  sampler_rot: None uses it unless a plan was
+    # installed as metro_plan, True / False (set by autotune.Autotuner.tune from
+    # its timings) decides.
+    sampler_rot = None
+
+    def rot_supported(self):
+        return 2 <= self.q <= 21 and 2 <= self.L <= 576 and self.nseq['main'] % 32 == 0
+
+    def sampler_kernel(self):
+        """The sampler runMCMC runs: 'rot' (mi3_metropolis_rot) or 'plan' (the
+        kernel and tiles of sampler_plan())."""
+        want = self.sampler_rot
+        if want is None:
+            want = not getattr(self, 'metro_plan', None)
+        return 'rot' if want and self.rot_supported() else 'plan'
+
     def sampler_plan(self):
-        """The plan runMCMC uses: ('skew', walkers_per_cta) or a
+        """The plan of the skewed-lane or row-streaming kernel, which runMCMC
+        uses when sampler_kernel() is 'plan': ('skew', walkers_per_cta) or a
         (walkers_per_cta, sites_per_chunk, stages) triple of the
         row-streaming kernel ((0, 0, 0): its built-in choice).  Set by
         autotune.Autotuner.tune as metro_plan; otherwise the skewed-lane
@@ -462,10 +515,17 @@ class MCMCGPU:
 
     def sampler_call(self, pos_offset, pos_ptr, nsteps, seq_ptr, rng_ptr, status_ptr, stream_ptr, betas=None,
                      plan=None):
-        """One sampler launch with the given plan (default: sampler_plan())
-        on caller-chosen buffers; J must already be unpacked for it."""
-        plan = tuple(plan) if plan else self.sampler_plan()
+        """One sampler launch with the given plan (default: the kernel of
+        sampler_kernel(); ('rot',) names the rotated one) on caller-chosen
+        buffers; J must already be unpacked for it."""
         N, L, q = self.nseq['main'], self.L, self.q
+        if not plan:
+            plan = ('rot',) if self.sampler_kernel() == 'rot' else self.sampler_plan()
+        plan = tuple(plan)
+        if plan[0] == 'rot':
+            _lib.call('mi3_metropolis_rot', self._ptr('Jrot'), rng_ptr, int(pos_offset), pos_ptr, int(nsteps), betas,
+                      self.beta, seq_ptr, N, L, q, 0, 0, status_ptr, stream_ptr)
+            return
         if plan[0] == 'skew':
             _lib.call('mi3_metropolis_skew', self._ptr('Jtiles'), rng_ptr, int(pos_offset), pos_ptr, int(nsteps),
                       betas, self.beta, seq_ptr, N, L, q, int(plan[1]), self.skew_replicas, status_ptr, stream_ptr)
@@ -868,9 +928,9 @@ class MCMCGPU:
     def getBuf(self, bufname, truncateLarge=True, wait_for=None):
         """Copy a device buffer to host; returns a FutureBuf
         (mcmcGPU.py:845-867)."""
-        if bufname == 'Junpacked' and self._unpacked_tiles and not self._unpacked_rows:
-            # the skewed-lane sampler unpacked J into the tiled layout only;
-            # build the rows a reader of 'Junpacked' expects from the same J
+        if bufname == 'Junpacked' and (self._unpacked_tiles or self._unpacked_rot) and not self._unpacked_rows:
+            # the sampler unpacked J into its own layout only; build the rows
+            # a reader of 'Junpacked' expects from the same J
             self.unpackJ(kind='rows')
         buftype, bufshape = self.buf_spec[bufname]
         dev = self.bufs[bufname]

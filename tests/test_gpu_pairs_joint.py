@@ -74,7 +74,8 @@ def test_residues_past_the_alphabet_count_as_the_last(cuda, q):
     res = []
     for s in (seqs, bad):
         cnt = empty((L * (L - 1) // 2, q * q), np.uint32)
-        _lib.call("mi3_bicounts", dev(oracle.pack_seqs(s)).data_ptr(), N, N, cnt.data_ptr(), L, q, stream())
+        dm = dev(oracle.pack_seqs(s))
+        _lib.call("mi3_bicounts", dm.data_ptr(), N, N, cnt.data_ptr(), L, q, stream())
         res.append(host(cnt, np.uint32))
     np.testing.assert_array_equal(res[1], res[0])
 
