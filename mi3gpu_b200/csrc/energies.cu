@@ -138,13 +138,14 @@ __device__ __forceinline__ double lane_energy(uint32_t jbase, const uint32_t (&r
 // Energies over joint sites (joint.cuh).  Bound by instruction issue at two
 // per gather (an add and a load) plus the sequence's offsets, with the
 // shared-memory pipe close behind; figures in joint.cuh.
-template <int B, int GI, int GJ, int T>
+template <int B, int GI, int GJ, int T, int QC>
 __global__ void __launch_bounds__(T, 1024 / T) k_energies_joint(const float *__restrict__ J,
                                                                const uint32_t *__restrict__ seq, uint32_t buflen,
                                                                uint32_t nseq, unsigned long long *acc, uint32_t L,
-                                                               uint32_t q, JointGeom g) {
+                                                               uint32_t q_any, JointGeom g) {
     extern __shared__ __align__(16) float js[];  // [cells][P], then the staged site pairs
     constexpr uint32_t P = B * B;
+    const uint32_t q = QC ? QC : q_any;
     const uint32_t qq = q * q, QI = joint_states(q, GI), QJ = joint_states(q, GJ);
     const uint32_t s = blockIdx.x % g.nslices, chunk = blockIdx.x / g.nslices;
     uint32_t bi, bj;
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_energies_joint(const float *__r
             for (uint32_t e = lane; e < qq; e += 32) raw[r * R + cc * S + e] = ok ? __ldg(&J[pair_index(i, j, L) * qq + e]) : 0.0f;
         }
         __syncthreads();
-        // each cell: the sum of its site pairs' couplings, rounded once
+        // each cell: the float sum of its (at most four) site pairs' couplings
         for (uint32_t c = warp; c < QI * QJ; c += nwarps) {
             const uint32_t A = c / QJ, Bc = c - A * QJ;
             uint32_t a[GI], b[GJ];
@@ -182,12 +183,13 @@ __global__ void __launch_bounds__(T, 1024 / T) k_energies_joint(const float *__r
 #pragma unroll
             for (uint32_t p = lane; p < P; p += 32) {
                 const float *src = raw + (p / B) * GI * R + (p % B) * GJ * S;
-                double v = 0.0;
+                float v[GI];
 #pragma unroll
-                for (int x = 0; x < GI; ++x)
-#pragma unroll
-                    for (int y = 0; y < GJ; ++y) v += (double)src[x * R + y * S + a[x] * q + b[y]];
-                js[c * P + p] = (float)v;
+                for (int x = 0; x < GI; ++x) {
+                    v[x] = src[x * R + a[x] * q + b[0]];
+                    if constexpr (GJ == 2) v[x] += src[x * R + S + a[x] * q + b[1]];
+                }
+                js[c * P + p] = GI == 1 ? v[0] : v[0] + v[GI - 1];
             }
         }
     }
@@ -272,7 +274,7 @@ static int launch_energies_joint(const float *J, const uint32_t *seq, uint32_t b
                                  unsigned long long *acc, uint32_t L, uint32_t q, cudaStream_t st) {
     const JointGeom g = joint_geom<C>(L, nseq);
     const size_t smem = joint_smem(q, C::B, C::GI, C::GJ);
-    auto kernel = k_energies_joint<C::B, C::GI, C::GJ, C::T>;
+    auto kernel = k_energies_joint<C::B, C::GI, C::GJ, C::T, C::QC>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const uint64_t nblk = (uint64_t)g.nslices * g.nchunks;
     if (nblk > 0x7fffffffull) return fail(MI3_ERR_ARG, "mi3_energies: grid too large");

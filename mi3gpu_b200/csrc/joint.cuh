@@ -28,9 +28,10 @@
 //
 // Measured against the pair-major tiling with lanes over pairs in full slices
 // only (Newton phases on one B200, l1z or l2z included):
-//   L=93  q=4  2^18  8 steps   10.0 -> 2.92 ms
-//   L=151 q=8  66048 8 steps   5.55 -> 3.58 ms
-//   L=232 q=21 2^20  3 steps   38.6 -> 36.8 ms (edge slices, packed adds, one
+//   L=93  q=4  2^18  8 steps   10.0 -> 2.37 ms (2.92 with the alphabet a
+//                              run-time value in the packing and splitting)
+//   L=151 q=8  66048 8 steps   5.55 -> 3.14 ms (3.58)
+//   L=232 q=21 2^20  3 steps   38.6 -> 36.7 ms (edge slices, packed adds, one
 //                              clamp test per word)
 #pragma once
 #include "tiling.cuh"
@@ -188,32 +189,37 @@ __device__ __forceinline__ void joint_sequences(const uint32_t *__restrict__ seq
 
 // Tile configuration of an alphabet: B joint sites per block, GI x GJ sites
 // per joint pair, T threads (1024 resident threads per SM at 64 registers,
-// so T = 1024 where one table fills the SM).
-template <int B_, int GI_, int GJ_, int T_>
+// so T = 1024 where one table fills the SM), and the alphabet QC where joint
+// states are packed and split, so that those divisions and sums unroll (0: any).
+// OVERHEAD: what building or splitting a CTA's table costs, in sequences.
+template <int B_, int GI_, int GJ_, int T_, int QC_>
 struct JointCfg {
-    static constexpr int B = B_, GI = GI_, GJ = GJ_, T = T_;
+    static constexpr int B = B_, GI = GI_, GJ = GJ_, T = T_, QC = QC_;
+    static constexpr uint32_t OVERHEAD = GI * GJ == 1 ? 2048 : 4096;
 };
 
 // Calls fn(JointCfg) for the alphabet; returns false when it has none.
 template <typename F>
 static bool joint_dispatch(uint32_t q, F &&fn) {
-    if (q == 1 || q == 9 || q == 10) fn(JointCfg<16, 1, 1, 512>());
-    else if (q == 2 || q == 3) fn(JointCfg<16, 2, 2, 512>());
-    else if (q == 4) fn(JointCfg<8, 2, 2, 512>());
-    else if (q == 5) fn(JointCfg<8, 2, 2, 1024>());
-    else if (q == 6 || q == 7) fn(JointCfg<8, 2, 1, 512>());
-    else if (q == 8) fn(JointCfg<8, 2, 1, 1024>());
-    else if (q >= 11 && q <= 21) fn(JointCfg<8, 1, 1, 512>());
+    if (q == 1 || q == 9 || q == 10) fn(JointCfg<16, 1, 1, 512, 0>());
+    else if (q == 2) fn(JointCfg<16, 2, 2, 512, 2>());
+    else if (q == 3) fn(JointCfg<16, 2, 2, 512, 3>());
+    else if (q == 4) fn(JointCfg<8, 2, 2, 512, 4>());
+    else if (q == 5) fn(JointCfg<8, 2, 2, 1024, 5>());
+    else if (q == 6) fn(JointCfg<8, 2, 1, 512, 6>());
+    else if (q == 7) fn(JointCfg<8, 2, 1, 512, 7>());
+    else if (q == 8) fn(JointCfg<8, 2, 1, 1024, 8>());
+    else if (q >= 11 && q <= 21) fn(JointCfg<8, 1, 1, 512, 0>());
     else return false;
     return true;
 }
 
+// All CTAs of a pass do the same work, so one wave will do.
 template <typename C>
-static JointGeom joint_geom(uint32_t L, uint32_t nseq, uint32_t max_chunk = 0xffffff00u,
-                            uint32_t overhead = PAIR_CTA_OVERHEAD) {
+static JointGeom joint_geom(uint32_t L, uint32_t nseq) {
     JointGeom g;
     joint_slices(L, C::B, C::GI, C::GJ, &g);
-    g.chunk = pick_chunk(g.nslices, nseq, 148 * (1024 / C::T), max_chunk, overhead);
+    g.chunk = pick_chunk(g.nslices, nseq, 148 * (1024 / C::T), 0xffffff00u, C::OVERHEAD, 1);
     g.nchunks = (nseq - 1) / g.chunk + 1;
     return g;
 }

@@ -128,22 +128,23 @@ __device__ __forceinline__ void hist_chunk(uint32_t *h, const uint32_t *__restri
 // pairs it counts; sums of a chunk's increments fit u32 (fixed_shift).  Bound by
 // instruction issue, two per (sequence, joint pair), and the shared-memory
 // reductions; figures in joint.cuh.
-template <int B, int GI, int GJ, int T, bool WEIGHTED>
+template <int B, int GI, int GJ, int T, int QC, bool WEIGHTED>
 __global__ void __launch_bounds__(T, 1024 / T) k_pairhist_joint(const uint32_t *__restrict__ seq, uint32_t buflen,
                                                                uint32_t nseq, const float *__restrict__ weights,
                                                                const unsigned int *__restrict__ wmax_bits,
-                                                               uint32_t *out, uint32_t L, uint32_t q, JointGeom g,
+                                                               uint32_t *out, uint32_t L, uint32_t q_any, JointGeom g,
                                                                uint64_t nbins) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t *h = reinterpret_cast<uint32_t *>(smem_raw);  // [cells][P], then the site pairs' bins
     constexpr uint32_t P = B * B;
+    const uint32_t q = QC ? QC : q_any;
     const uint32_t qq = q * q, QJ = joint_states(q, GJ), ncell = joint_states(q, GI) * QJ;
     const uint32_t s = blockIdx.x % g.nslices, chunk = blockIdx.x / g.nslices;
     uint32_t bi, bj;
     joint_coords<GI, GJ>(s, g.nbJ, bi, bj);
     const uint32_t i0 = bi * (B * GI), j0 = bj * (B * GJ);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = T / 32;
-    for (uint32_t k = threadIdx.x; k < ncell * P; k += T) h[k] = 0u;
+    for (uint32_t k = threadIdx.x; k < ncell * P / 4; k += T) reinterpret_cast<uint4 *>(h)[k] = make_uint4(0, 0, 0, 0);
     float scale = 1.0f;
     if constexpr (WEIGHTED) scale = ldexpf(1.0f, fixed_shift(__uint_as_float(*wmax_bits), g.chunk));
     __syncthreads();
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_pairhist_joint(const uint32_t *
     } else {
         uint32_t *raw = h + joint_table(q, B, GI, GJ);
         const uint32_t S = joint_stage_pair(q, GJ), R = joint_stage_row(q, B, GJ);
-        const uint32_t rowother = GI == 2 ? q : 1, colother = GJ == 2 ? q : 1;
+        constexpr uint32_t rowother = GI == 2 ? QC : 1, colother = GJ == 2 ? QC : 1;
         // bin (a, b) of sub-pair (x, y): the joint bins over the other residues
         for (uint32_t t = warp; t < GI * GJ * qq; t += nwarps) {
             const uint32_t xy = t / qq, e = t - xy * qq, a = e / q, b = e - a * q;
@@ -196,7 +197,9 @@ __global__ void __launch_bounds__(T, 1024 / T) k_pairhist_joint(const uint32_t *
 #pragma unroll
             for (uint32_t p = lane; p < P; p += 32) {
                 uint32_t v = 0;
+#pragma unroll
                 for (uint32_t u = 0; u < rowother; ++u)
+#pragma unroll
                     for (uint32_t w = 0; w < colother; ++w) v += h[((A0 + u * dA) * QJ + B0 + w * dB) * P + p];
                 raw[((p / B) * GI + x) * R + ((p % B) * GJ + y) * S + e] = v;
             }
@@ -529,7 +532,7 @@ static int launch_pairhist_joint(const uint32_t *seq, uint32_t buflen, uint32_t 
         g.nchunks = (nseq - 1) / g.chunk + 1;
     }
     const size_t smem = joint_smem(q, C::B, C::GI, C::GJ);
-    auto kernel = k_pairhist_joint<C::B, C::GI, C::GJ, C::T, WEIGHTED>;
+    auto kernel = k_pairhist_joint<C::B, C::GI, C::GJ, C::T, C::QC, WEIGHTED>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const uint64_t nblk = (uint64_t)g.nslices * g.nchunks;
     if (nblk > 0x7fffffffull) return fail(MI3_ERR_ARG, "pair histogram: grid too large");

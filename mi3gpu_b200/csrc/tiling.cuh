@@ -54,12 +54,12 @@ inline uint32_t pick_block(uint32_t q, size_t budget, uint32_t max_b = 32) {
 // (Targeting a fixed number of CTAs instead left last waves nearly empty:
 // 2080 CTAs = 7.03 waves at L=512, q=21, 2^18 sequences.)
 // For each number of waves only the largest nchunks that fits it is tried,
-// from PAIR_MIN_WAVES on: slices differ in cost, which several CTAs per slot
-// even out.
+// from min_waves on (PAIR_MIN_WAVES where slices differ in cost, which several
+// CTAs per slot even out).
 constexpr uint32_t PAIR_RESIDENT = 148 * 2, PAIR_CTA_OVERHEAD = 2048, PAIR_MIN_CHUNK = 1024, PAIR_MIN_WAVES = 3;
 
 inline uint32_t pick_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident, uint32_t max_chunk,
-                           uint32_t overhead) {
+                           uint32_t overhead, uint32_t min_waves) {
     const uint32_t min_chunk = std::min(PAIR_MIN_CHUNK, max_chunk);
     const uint32_t least = (nseq - 1) / max_chunk + 1;  // chunks that max_chunk asks for
     const uint32_t most = std::max(least, (nseq - 1) / min_chunk + 1);
@@ -67,7 +67,7 @@ inline uint32_t pick_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident, u
     uint32_t pick = chunk_of(least);
     uint64_t best = ~0ull;
     const uint32_t w0 = (uint32_t)(((uint64_t)nslices * least + resident - 1) / resident);
-    for (uint32_t w = std::max(w0, PAIR_MIN_WAVES); w < w0 + 24; ++w) {
+    for (uint32_t w = std::max(w0, min_waves); w < w0 + 24; ++w) {
         const uint64_t fit = (uint64_t)w * resident / nslices;
         const uint32_t chunk = chunk_of((uint32_t)std::min<uint64_t>(std::max<uint64_t>(fit, least), most));
         const uint64_t cost = w * ((uint64_t)chunk + overhead);
@@ -80,13 +80,12 @@ inline uint32_t pick_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident, u
     return pick;
 }
 
-inline SliceGeom make_geom(uint32_t L, uint32_t B, uint32_t nseq, uint32_t max_chunk = 0xffffff00u,
-                           uint32_t overhead = PAIR_CTA_OVERHEAD) {
+inline SliceGeom make_geom(uint32_t L, uint32_t B, uint32_t nseq) {
     SliceGeom g;
     g.B = B;
     g.nb = (L + B - 1) / B;
     g.nslices = g.nb * (g.nb + 1) / 2;
-    g.chunk = pick_chunk(g.nslices, nseq, PAIR_RESIDENT, max_chunk, overhead);
+    g.chunk = pick_chunk(g.nslices, nseq, PAIR_RESIDENT, 0xffffff00u, PAIR_CTA_OVERHEAD, PAIR_MIN_WAVES);
     g.nchunks = (nseq - 1) / g.chunk + 1;
     return g;
 }

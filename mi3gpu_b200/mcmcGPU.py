@@ -573,11 +573,12 @@ class MCMCGPU:
 
     # ------------------------------------------------------------ statistics
     # alphabet sizes for which the tcgen05 one-hot GEMM counts beat the
-    # shared-memory histogram when nothing was tuned (measured on B200 at
-    # 2^18 walkers against the lanes-over-pairs histogram: 2.5x at q=4, 2.2x
-    # at q=5, 1.8x at q=6, a tie at q=8 and at 2^14 walkers, slower from
-    # q=12 on); both give identical integers.
-    TENSOR_COUNT_Q = range(4, 7)
+    # shared-memory histogram when nothing was tuned: none since the histogram
+    # counts up to four site pairs per add (B200, tensor cores against it: 108
+    # / 71 us at L=93 q=4 2^18, 149 / 89 us at L=99 q=5 2^18, 202 / 122 us at
+    # L=99 q=6 2^18, 326 / 278 us at L=300 q=4 2^17, 23 / 12 us at L=48 q=4
+    # 2^14); both give identical integers, and the autotuner times both.
+    TENSOR_COUNT_Q = range(0)
     # the same for the weighted bimarginals (three byte-plane integer GEMMs
     # against the shared-memory fixed-point histogram, identical results):
     # since the histogram visits pairs with lanes over pairs it is as fast at
