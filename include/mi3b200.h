@@ -458,6 +458,33 @@ int mi3_weights_fused(float ref_E, const float *dE, float *weights, uint32_t n, 
                       float *out2, double *out2_f64, void *workspace, size_t ws_bytes,
                       void *stream);
 
+/* One quasi-Newton step on fixed sequences (NewtonSteps.py:217-246): dJ takes
+ * mi3_update_j and, with reg 1 or 2, mi3_reg_l1z or mi3_reg_l2z; energies =
+ * those of dJ; mi3_weights_fused with ref_E; then bi = mi3_weighted_marg and
+ * mi3_renormalize_bimarg.  The same kernels as the separate calls, so the same
+ * bits.  host_out (4 doubles in pinned host memory) receives {sum w, sum w^2,
+ * min(0, min dE), *status} and `event` (a cudaEvent_t) is recorded behind that,
+ * before the weighted pass, so that the host can decide on the next step while
+ * it runs.  The argument block stays valid for any number of calls while its
+ * buffers do. */
+typedef struct {
+    const float *bi_target;
+    float *bi, *dJ;
+    const float *J;
+    const uint32_t *seqmem;
+    uint32_t buflen, nseq, L, q;
+    float gamma, pc, lJ;
+    int32_t reg;
+    float *energies, *weights, *minout, *weight_stats;
+    double *weight_stats64;
+    void *ws_energies, *ws_reduce, *ws_wmarg;
+    uint64_t ws_energies_bytes, ws_reduce_bytes, ws_wmarg_bytes;
+    const int32_t *status;
+    double *host_out;
+    void *event;
+} mi3_newton_args;
+int mi3_newton_step(const mi3_newton_args *args, float ref_E, void *stream);
+
 /* ------------------------------------------------ learned proposal (MADE)
  * No counterpart in the reference: a masked autoregressive network over
  * L sites x q residues (two hidden layers of H units) trained on sampled

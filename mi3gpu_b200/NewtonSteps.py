@@ -70,6 +70,19 @@ def singleNewton(bimarg, gamma, param, gpus):
     return gpus.head_gpu.getBuf('J')[0].read()
 
 
+def _neff_line(i, wsum, wsum2, lastNeff, N0, Nfrac, log):
+    """A step's Neff, logged as the reference does (NewtonSteps.py:234-246):
+    (Neff, Neff last logged, whether the steps end here)."""
+    Neff = np.float64(wsum) ** 2 / np.float64(wsum2)
+    if i % 64 == 0 or abs(lastNeff - Neff) / N0 > 0.05 or Neff < Nfrac * N0:
+        log(f"J-step {i: 5d}   Neff: {Neff:.1f}   ({Neff / N0 * 100:.1f}% of {N0})")
+        lastNeff = Neff
+    if Neff < Nfrac * N0:
+        log(f"Ending coupling updates because Neff/N < {Nfrac:.2f}")
+        return Neff, lastNeff, True
+    return Neff, lastNeff, False
+
+
 def iterNewton(param, bimarg_model, gpus, log, fused=False):
     """Zwanzig-reweighted quasi-Newton steps until Neff < fracNeff*N
     (NewtonSteps.py:159-268).  Returns (steps, trialJ, predicted bimarg).
@@ -128,7 +141,19 @@ def iterNewton(param, bimarg_model, gpus, log, fused=False):
 
     lastNeff = 2 * N0
     i = 0
+    # one native call per step where the device group has it (the same
+    # kernels; fused or not gives the same values)
+    step = None
+    if param.beta is None and hasattr(gpus, 'newtonStepper'):
+        step = gpus.newtonStepper(gamma, pc, param.reg, tuple(param.regarg or ()), seqbuf)
     for i in range(newtonSteps):
+        if step is not None:
+            wsum, wsum2, mindE = step(ref_dE)
+            Neff, lastNeff, done = _neff_line(i, wsum, wsum2, lastNeff, N0, Nfrac, log)
+            if done:
+                break
+            ref_dE = mindE
+            continue
         gpus.updateJ(gamma, pc)
         if param.reg is not None:
             gpus.reg(param.reg, (gamma, pc,) + tuple(param.regarg))
@@ -150,12 +175,8 @@ def iterNewton(param, bimarg_model, gpus, log, fused=False):
         gpus.merge_bimarg()
 
         wsum, wsum2 = (np.sum(x) for x in zip(*(w.read() for w in w_fut)))
-        Neff = wsum ** 2 / wsum2
-        if i % 64 == 0 or abs(lastNeff - Neff) / N0 > 0.05 or Neff < Nfrac * N0:
-            log(f"J-step {i: 5d}   Neff: {Neff:.1f}   ({Neff / N0 * 100:.1f}% of {N0})")
-            lastNeff = Neff
-        if Neff < Nfrac * N0:
-            log(f"Ending coupling updates because Neff/N < {Nfrac:.2f}")
+        Neff, lastNeff, done = _neff_line(i, wsum, wsum2, lastNeff, N0, Nfrac, log)
+        if done:
             break
         ref_dE = np.min([x.read()[()] for x in mindE_fut])
 

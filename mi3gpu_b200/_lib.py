@@ -11,6 +11,17 @@ LIB_PATH = Path(__file__).resolve().parent / "libmi3b200.so"
 c = ctypes
 _vp, _u32, _u64, _f32, _i32 = c.c_void_p, c.c_uint32, c.c_uint64, c.c_float, c.c_int32
 
+class NewtonArgs(c.Structure):
+    """mi3_newton_args of include/mi3b200.h."""
+    _fields_ = [("bi_target", _vp), ("bi", _vp), ("dJ", _vp), ("J", _vp), ("seqmem", _vp),
+                ("buflen", _u32), ("nseq", _u32), ("L", _u32), ("q", _u32),
+                ("gamma", _f32), ("pc", _f32), ("lJ", _f32), ("reg", _i32),
+                ("energies", _vp), ("weights", _vp), ("minout", _vp), ("weight_stats", _vp), ("weight_stats64", _vp),
+                ("ws_energies", _vp), ("ws_reduce", _vp), ("ws_wmarg", _vp),
+                ("ws_energies_bytes", _u64), ("ws_reduce_bytes", _u64), ("ws_wmarg_bytes", _u64),
+                ("status", _vp), ("host_out", _vp), ("event", _vp)]
+
+
 # name -> (restype, argtypes); mirrors include/mi3b200.h
 SIGNATURES = {
     "mi3_last_error": (c.c_char_p, []),
@@ -74,6 +85,7 @@ SIGNATURES = {
     "mi3_weight_stats_workspace": (c.c_size_t, [_u32]),
     "mi3_weight_stats": (c.c_int, [_vp, _u32, _vp, _vp, _vp, c.c_size_t, _vp]),
     "mi3_weights_fused": (c.c_int, [_f32, _vp, _vp, _u32, _vp, _vp, _vp, _vp, c.c_size_t, _vp]),
+    "mi3_newton_step": (c.c_int, [c.POINTER(NewtonArgs), _f32, _vp]),
     "mi3_add_float_bufs": (c.c_int, [_vp, _vp, _u32, _vp]),
     "mi3_weights_fused_dev": (c.c_int, [_vp, _vp, _vp, _u32, _vp, _vp, _vp, _vp, c.c_size_t, _vp]),
     "mi3_capture_begin": (c.c_int, [_vp]),

@@ -55,6 +55,9 @@ class RankNode(GPU_node):
     def _backend(self):
         return dist.get_backend(self.group)
 
+    def newtonStepper(self, *args):
+        return None  # every step merges bimarginals and weight sums over the ranks
+
     # -------------------------------------------------------- shape
     @property
     def head_gpu(self):

@@ -884,6 +884,45 @@ class MCMCGPU:
         self.unpackedJ = None
         return self.logevt('reg_l2z', s)
 
+    def newtonStepper(self, gamma, pc, reg, regarg, seqbufname='main'):
+        """iterNewton's step as one native call (mi3_newton_step): a function
+        of the reference energy that returns the step's (sum w, sum w^2,
+        min(0, min dE)), with the step's weighted bimarginals still being
+        computed on the device.  None where the step needs what that call does
+        not do: profiled commands, other regularizers, the consensus or
+        tensor-core kernels."""
+        self.require('Jstep')
+        if (self.profile or reg not in (None, 'l1z', 'l2z') or (reg and len(regarg) != 1)
+                or getattr(self, 'consEnergies', False)
+                or getattr(self, 'consWmarg', False) or getattr(self, 'wmarg_kernel', None) == 'tc'
+                or self.q in self.TENSOR_WMARG_Q):
+            return None
+        nseq, buflen = self._span(seqbufname)
+        host = torch.empty(4, dtype=torch.float64, pin_memory=True)
+        evt = torch.cuda.Event()
+        evt.record(self.stream)  # creates the event the library records
+        args = _lib.NewtonArgs(
+            bi_target=self._ptr('bi target'), bi=self._ptr('bi'), dJ=self._ptr('dJ'), J=self._ptr('J'),
+            seqmem=self.seqbufs[seqbufname].data_ptr(), buflen=buflen, nseq=nseq, L=self.L, q=self.q, gamma=gamma,
+            pc=pc, lJ=float(regarg[0]) if reg else 0.0, reg={None: 0, 'l1z': 1, 'l2z': 2}[reg],
+            energies=self.Ebufs[seqbufname].data_ptr(), weights=self._ptr(self._wbufname(seqbufname)),
+            minout=self._ptr('minout'), weight_stats=self._ptr('weightstats'),
+            weight_stats64=self._ptr('weightstats64'), ws_energies=self._ptr('ws energies'),
+            ws_reduce=self._ptr('ws reduce'), ws_wmarg=self._ptr('ws wmarg'),
+            ws_energies_bytes=self._wsbytes('ws energies'), ws_reduce_bytes=self._wsbytes('ws reduce'),
+            ws_wmarg_bytes=self._wsbytes('ws wmarg'), status=self._ptr('status'), host_out=host.data_ptr(),
+            event=evt.cuda_event)
+        out = host.numpy()
+
+        def step(ref_E):
+            self.unpackedJ = None if reg else False  # as updateJ and reg_* leave it
+            _lib.call('mi3_newton_step', args, float(ref_E), self._s)
+            evt.synchronize()
+            if out[3] != 0:
+                self._check_status()
+            return float(out[0]), float(out[1]), np.float32(out[2])
+        return step
+
     def _reg(self, entry, name, *args, lambdas=False):
         self.require('Jstep')
         s = self._begin()

@@ -251,6 +251,13 @@ class GPU_node:
         for gpu in self.gpus:
             gpu.updateJ(gamma, pc, Jbuf)
 
+    def newtonStepper(self, *args):
+        """One device: its newtonStepper (merge_bimarg is then the step's
+        renormalisation); None with several, whose results are merged."""
+        if self.ngpus != 1 or not hasattr(self.gpus[0], 'newtonStepper'):
+            return None
+        return self.gpus[0].newtonStepper(*args)
+
     def reg(self, name, param):
         meth = 'reg_{}'.format(name)
         for gpu in self.gpus:
