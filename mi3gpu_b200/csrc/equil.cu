@@ -11,9 +11,9 @@
 // |r|, p > 0.02 is the same as |r| < r_crit with r_crit = t_c / sqrt(n - 2 +
 // t_c^2), t_c the upper 1% point of that t distribution -- a number the host
 // computes once per n.  Here:
-//   mi3_rank_average   ranks of n floats (bitonic sort of (key, index)
-//                      pairs, tie runs found by two prefix scans, average
-//                      rank scattered back to the input order);
+//   mi3_rank_average   ranks of n floats (radix sort of (key, index) pairs,
+//                      tie runs found by binary search, average rank
+//                      scattered back to the input order);
 //   mi3_rank_corr      Pearson r of two rank vectors in FP64 (fixed-order
 //                      reduction, so the result is deterministic);
 //   mi3_equil_decide   the verdict |r1| < r_crit and |r2| < r_crit as an
@@ -25,10 +25,6 @@
 
 namespace mi3 {
 
-constexpr uint32_t RK_THREADS = 1024;
-constexpr uint32_t RK_TILE = 2 * RK_THREADS;  // elements sorted per block in shared memory
-constexpr uint32_t RK_PAD_KEY = 0xffffffffu;   // sorts after every finite float
-
 // Order-preserving map float -> uint32 (finite inputs); -0 and +0 are one
 // value, as for a float comparison.
 __device__ __forceinline__ uint32_t float_key(float x) {
@@ -36,166 +32,135 @@ __device__ __forceinline__ uint32_t float_key(float x) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// (key, index) pairs compare by key, then index: a total order.
-__device__ __forceinline__ bool pair_gt(uint32_t ka, uint32_t va, uint32_t kb, uint32_t vb) {
-    return ka > kb || (ka == kb && va > vb);
-}
+// Least-significant-digit radix sort, 8 bits a pass.  A pass is one kernel: each
+// CTA sorts a tile of RK_TILE pairs stably by its digit and finds where each
+// digit's run goes from all CTAs' digit counts, which the pass before it made
+// (count[tile][digit], 1 KB per tile, read by every CTA from L2).  So a sort is
+// six launches, tie handling included, whatever n; the bitonic network it
+// replaces took 44 at n = 2^18, most of them 3 us long.  Call times, before and
+// now: 103 and 68 us at n = 2^14, 235 and 84 us at 2^18, 514 and 172 us at 2^20.
+// A pass is bound by its latencies: the reads of the counts, then 16 rounds of
+// matching.
+constexpr uint32_t RK_THREADS = 256, RK_WARPS = RK_THREADS / 32, RK_PER = 16;
+constexpr uint32_t RK_TILE = RK_THREADS * RK_PER, RK_DIGITS = 256;
 
-__device__ __forceinline__ void cmp_swap(uint32_t &ka, uint32_t &va, uint32_t &kb, uint32_t &vb, bool asc) {
-    if (pair_gt(ka, va, kb, vb) == asc) {
-        uint32_t t = ka;
-        ka = kb;
-        kb = t;
-        t = va;
-        va = vb;
-        vb = t;
-    }
-}
-
-// The bitonic network's steps (k, j) with j < RK_TILE, for one tile in
-// shared memory.  kmax = 0: every k from 2 to RK_TILE (the first pass over
-// fresh input); otherwise only k = kmax (the tail of a global merge).
-__device__ void tile_network(uint32_t *sk, uint32_t *sv, uint32_t base, uint32_t kmax) {
-    const uint32_t k0 = kmax ? kmax : 2, k1 = kmax ? kmax : RK_TILE;
-    for (uint32_t k = k0; k <= k1; k <<= 1) {
-        for (uint32_t j = (k >> 1) < (RK_TILE >> 1) ? (k >> 1) : (RK_TILE >> 1); j > 0; j >>= 1) {
-            const uint32_t t = threadIdx.x;
-            const uint32_t i = 2 * j * (t / j) + (t % j), l = i + j;
-            const bool asc = ((base + i) & k) == 0;
-            cmp_swap(sk[i], sv[i], sk[l], sv[l], asc);
-            __syncthreads();
-        }
-    }
-}
-
-__global__ void __launch_bounds__(RK_THREADS) k_rank_tiles(const float *__restrict__ x, uint32_t n,
-                                                           uint32_t *keys, uint32_t *vals) {
-    __shared__ uint32_t sk[RK_TILE], sv[RK_TILE];
-    const uint32_t base = blockIdx.x * RK_TILE;
-    for (uint32_t i = threadIdx.x; i < RK_TILE; i += RK_THREADS) {
-        const uint32_t g = base + i;
-        sk[i] = g < n ? float_key(x[g]) : RK_PAD_KEY;
-        sv[i] = g;
-    }
+__global__ void __launch_bounds__(RK_THREADS) k_rank_count(const float *__restrict__ x, uint32_t n, uint32_t *count) {
+    __shared__ uint32_t c[RK_DIGITS];
+    c[threadIdx.x] = 0;
     __syncthreads();
-    tile_network(sk, sv, base, 0);
-    for (uint32_t i = threadIdx.x; i < RK_TILE; i += RK_THREADS) {
-        keys[base + i] = sk[i];
-        vals[base + i] = sv[i];
-    }
-}
-
-// One global step (k, j >= RK_TILE): thread t compares pair (i, i + j).
-__global__ void k_rank_global(uint32_t *keys, uint32_t *vals, uint32_t k, uint32_t j, uint32_t half) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= half) return;
-    const uint32_t i = 2 * j * (t / j) + (t % j), l = i + j;
-    uint32_t ka = keys[i], va = vals[i], kb = keys[l], vb = vals[l];
-    cmp_swap(ka, va, kb, vb, (i & k) == 0);
-    keys[i] = ka;
-    vals[i] = va;
-    keys[l] = kb;
-    vals[l] = vb;
-}
-
-// Steps (k, j < RK_TILE) of a merge stage k > RK_TILE, one tile per block.
-__global__ void __launch_bounds__(RK_THREADS) k_rank_merge(uint32_t *keys, uint32_t *vals, uint32_t k) {
-    __shared__ uint32_t sk[RK_TILE], sv[RK_TILE];
     const uint32_t base = blockIdx.x * RK_TILE;
-    for (uint32_t i = threadIdx.x; i < RK_TILE; i += RK_THREADS) {
-        sk[i] = keys[base + i];
-        sv[i] = vals[base + i];
-    }
-    __syncthreads();
-    tile_network(sk, sv, base, k);
-    for (uint32_t i = threadIdx.x; i < RK_TILE; i += RK_THREADS) {
-        keys[base + i] = sk[i];
-        vals[base + i] = sv[i];
-    }
-}
-
-// Prefix maximum over positions (two levels: a block scan with its total,
-// then the totals, then the carry) of: p where a run of equal sorted keys
-// starts, else 0 (REV false: gives each position its run's first index);
-// or, counting positions p' from the end, p' where a run ends (REV true:
-// gives its run's last index as n - 1 - result).
-constexpr uint32_t SC_THREADS = 1024, SC_PER = 4, SC_TILE = SC_THREADS * SC_PER;
-
-template <bool REV>
-__device__ __forceinline__ uint32_t run_mark(const uint32_t *keys, uint32_t n, uint32_t p) {
-    // REV: p counts from the end; a run "starts" there when the next key
-    // (towards the end) differs
-    const uint32_t q = REV ? n - 1 - p : p;
-    const bool edge = REV ? (q == n - 1 || keys[q] != keys[q + 1]) : (q == 0 || keys[q] != keys[q - 1]);
-    return edge ? p : 0u;
-}
-
-template <bool REV>
-__global__ void __launch_bounds__(SC_THREADS) k_scan_max_local(const uint32_t *__restrict__ keys, uint32_t n,
-                                                               uint32_t *out, uint32_t *agg) {
-    __shared__ uint32_t wtot[SC_THREADS / 32];
-    const uint32_t base = blockIdx.x * SC_TILE + threadIdx.x * SC_PER;
-    uint32_t v[SC_PER], run = 0;
 #pragma unroll
-    for (uint32_t e = 0; e < SC_PER; ++e) {
-        const uint32_t p = base + e;
-        v[e] = p < n ? run_mark<REV>(keys, n, p) : 0u;
-        run = max(run, v[e]);
-        v[e] = run;
+    for (uint32_t e = 0; e < RK_PER; ++e) {
+        const uint32_t i = base + e * RK_THREADS + threadIdx.x;
+        if (i < n) atomicAdd(&c[float_key(x[i]) & 255u], 1u);
     }
-    // inclusive max-scan of the thread totals across the block
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = run;
+    __syncthreads();
+    count[blockIdx.x * RK_DIGITS + threadIdx.x] = c[threadIdx.x];
+}
+
+// One pass by bits [shift, shift + 8): the pairs of (x, index) if FIRST, else of
+// (keys_in, vals_in), to keys_out / vals_out; counts the next digit of what it
+// writes into next (nullable, zeroed).
+template <bool FIRST>
+__global__ void __launch_bounds__(RK_THREADS) k_rank_pass(const float *__restrict__ x,
+                                                          const uint32_t *__restrict__ keys_in,
+                                                          const uint32_t *__restrict__ vals_in, uint32_t n,
+                                                          uint32_t shift, const uint32_t *__restrict__ count,
+                                                          uint32_t *next, uint32_t *keys_out, uint32_t *vals_out) {
+    __shared__ uint32_t cnt[RK_WARPS][RK_DIGITS], scan[RK_DIGITS];
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    for (uint32_t w = 0; w < RK_WARPS; ++w) cnt[w][t] = 0;
+    // digit t: its total, and its count in the tiles before this one
+    uint32_t total = 0, before = 0;
+#pragma unroll 8
+    for (uint32_t b = 0; b < gridDim.x; ++b) {
+        const uint32_t v = __ldg(&count[b * RK_DIGITS + t]);
+        total += v;
+        before += b < blockIdx.x ? v : 0u;
+    }
+    __syncthreads();
+
+    // stable rank of each pair among its warp's pairs of the same digit: the
+    // warp takes RK_PER rounds of 32 neighbouring pairs
+    const uint32_t seg = blockIdx.x * RK_TILE + warp * (RK_PER * 32);
+    uint32_t key[RK_PER], val[RK_PER], rank[RK_PER];
+#pragma unroll
+    for (uint32_t e = 0; e < RK_PER; ++e) {
+        const uint32_t i = seg + e * 32 + lane;
+        key[e] = i < n ? (FIRST ? float_key(x[i]) : keys_in[i]) : 0u;
+        val[e] = FIRST || i >= n ? i : vals_in[i];
+    }
+#pragma unroll
+    for (uint32_t e = 0; e < RK_PER; ++e) {
+        const bool in = seg + e * 32 + lane < n;
+        const uint32_t live = __ballot_sync(0xffffffffu, in), d = (key[e] >> shift) & 255u;
+        if (in) {
+            const uint32_t same = __match_any_sync(live, d), mine = __popc(same & ((1u << lane) - 1u));
+            rank[e] = cnt[warp][d] + mine;
+            __syncwarp(live);
+            if (mine == 0) cnt[warp][d] += __popc(same);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    // exclusive scan of the digit totals; each warp's share of its digits
+    uint32_t inc = total;
 #pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x = max(x, y);
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
     }
-    if (lane == 31) wtot[warp] = x;
+    if (lane == 31) scan[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < SC_THREADS / 32 ? wtot[lane] : 0u;
-#pragma unroll
-        for (uint32_t o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w = max(w, y);
-        }
-        if (lane < SC_THREADS / 32) wtot[lane] = w;
+    uint32_t start = inc - total + before;
+    for (uint32_t w = 0; w < warp; ++w) start += scan[w];
+    for (uint32_t w = 0; w < RK_WARPS; ++w) {
+        const uint32_t c = cnt[w][t];
+        cnt[w][t] = start;
+        start += c;
     }
     __syncthreads();
-    uint32_t carry = __shfl_up_sync(0xffffffffu, x, 1);
-    if (lane == 0) carry = 0;
-    if (warp > 0) carry = max(carry, wtot[warp - 1]);
 #pragma unroll
-    for (uint32_t e = 0; e < SC_PER; ++e)
-        if (base + e < n) out[base + e] = max(v[e], carry);
-    if (threadIdx.x == 0) agg[blockIdx.x] = wtot[SC_THREADS / 32 - 1];  // the block's maximum
-}
-
-// Exclusive max-scan of the block totals (one block; nb <= SC_THREADS * SC_PER).
-__global__ void __launch_bounds__(SC_THREADS) k_scan_max_aggs(uint32_t *agg, uint32_t nb) {
-    if (threadIdx.x != 0) return;
-    uint32_t run = 0;
-    for (uint32_t b = 0; b < nb; ++b) {
-        const uint32_t t = agg[b];
-        agg[b] = run;
-        run = max(run, t);
+    for (uint32_t e = 0; e < RK_PER; ++e) {
+        if (seg + e * 32 + lane >= n) continue;
+        const uint32_t at = cnt[warp][(key[e] >> shift) & 255u] + rank[e];
+        keys_out[at] = key[e];
+        vals_out[at] = val[e];
+        if (next) atomicAdd(&next[at / RK_TILE * RK_DIGITS + ((key[e] >> (shift + 8)) & 255u)], 1u);
     }
-}
-
-__global__ void k_scan_max_apply(uint32_t *out, uint32_t n, const uint32_t *__restrict__ agg) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) out[p] = max(out[p], agg[p / SC_TILE]);
 }
 
 // rank (1-based, average over the tie run [lo, hi]) scattered to the input
-// order
-__global__ void k_rank_scatter(const uint32_t *__restrict__ vals, const uint32_t *__restrict__ lo,
-                               const uint32_t *__restrict__ hirev, uint32_t n, float *ranks) {
+// order; a run's ends by binary search in the sorted keys
+__global__ void k_rank_scatter(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint32_t n,
+                               float *ranks) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
-    const uint32_t a = lo[p], b = n - 1 - hirev[n - 1 - p];
-    ranks[vals[p]] = 0.5f * (float)(a + b) + 1.0f;  // exact: a + b < 2^24
+    const uint32_t k = keys[p];
+    uint32_t lo = p, hi = p;
+    if (p > 0 && keys[p - 1] == k) {
+        uint32_t a = 0, b = p - 1;  // first index with this key is in [a, b]
+        while (a < b) {
+            const uint32_t m = (a + b) / 2;
+            if (keys[m] < k)
+                a = m + 1;
+            else
+                b = m;
+        }
+        lo = a;
+    }
+    if (p + 1 < n && keys[p + 1] == k) {
+        uint32_t a = p + 1, b = n - 1;  // last index with this key is in [a, b]
+        while (a < b) {
+            const uint32_t m = (a + b + 1) / 2;
+            if (keys[m] > k)
+                b = m - 1;
+            else
+                a = m;
+        }
+        hi = a;
+    }
+    ranks[vals[p]] = 0.5f * (float)(lo + hi) + 1.0f;  // exact: lo + hi < 2^24
 }
 
 // Pearson correlation of two rank vectors: per-block FP64 partial sums of
@@ -245,21 +210,15 @@ __global__ void k_equil_decide(const double *r1, const double *r2, double rcrit,
     *flag = (a < rcrit && b < rcrit) ? 1 : 0;  // false for NaN
 }
 
-static uint32_t pow2_at_least(uint32_t n) {
-    uint32_t p = RK_TILE;
-    while (p < n) p <<= 1;
-    return p;
-}
-
 }  // namespace mi3
 
 using namespace mi3;
 
 extern "C" size_t mi3_rank_workspace(uint32_t n) {
     if (n == 0 || n >= (1u << 23)) return 0;
-    const size_t P = pow2_at_least(n);
-    const size_t nb = (n + SC_TILE - 1) / SC_TILE;
-    return 2 * P * 4 + 2 * (size_t)n * 4 + 256 + nb * 4;
+    // two key and two index arrays, one table of digit counts per pass
+    const size_t nb = (n + RK_TILE - 1) / RK_TILE;
+    return 4 * (size_t)n * 4 + 4 * nb * RK_DIGITS * 4;
 }
 
 extern "C" int mi3_rank_average(const float *x, uint32_t n, float *ranks, void *workspace, size_t ws_bytes,
@@ -269,27 +228,17 @@ extern "C" int mi3_rank_average(const float *x, uint32_t n, float *ranks, void *
     if (ws_bytes < mi3_rank_workspace(n)) return fail(MI3_ERR_WORKSPACE, "mi3_rank_average: workspace too small");
     if (!aligned(workspace, 16)) return fail(MI3_ERR_ALIGN, "mi3_rank_average: workspace must be 16B aligned");
     cudaStream_t st = as_stream(stream);
-    const uint32_t P = pow2_at_least(n);
-    uint32_t *keys = reinterpret_cast<uint32_t *>(workspace);
-    uint32_t *vals = keys + P;
-    uint32_t *lo = vals + P;
-    uint32_t *hirev = lo + n;
-    uint32_t *agg = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(hirev + n) + 256);
-    k_rank_tiles<<<P / RK_TILE, RK_THREADS, 0, st>>>(x, n, keys, vals);
-    const uint32_t half = P / 2;
-    for (uint32_t k = 2 * RK_TILE; k <= P; k <<= 1) {
-        for (uint32_t j = k >> 1; j >= RK_TILE; j >>= 1)
-            k_rank_global<<<(half + 255) / 256, 256, 0, st>>>(keys, vals, k, j, half);
-        k_rank_merge<<<P / RK_TILE, RK_THREADS, 0, st>>>(keys, vals, k);
-    }
-    const uint32_t nb = (n + SC_TILE - 1) / SC_TILE;
-    k_scan_max_local<false><<<nb, SC_THREADS, 0, st>>>(keys, n, lo, agg);
-    k_scan_max_aggs<<<1, 32, 0, st>>>(agg, nb);
-    k_scan_max_apply<<<(n + 255) / 256, 256, 0, st>>>(lo, n, agg);
-    k_scan_max_local<true><<<nb, SC_THREADS, 0, st>>>(keys, n, hirev, agg);
-    k_scan_max_aggs<<<1, 32, 0, st>>>(agg, nb);
-    k_scan_max_apply<<<(n + 255) / 256, 256, 0, st>>>(hirev, n, agg);
-    k_rank_scatter<<<(n + 255) / 256, 256, 0, st>>>(vals, lo, hirev, n, ranks);
+    const uint32_t nb = (n + RK_TILE - 1) / RK_TILE, table = nb * RK_DIGITS;
+    uint32_t *count = reinterpret_cast<uint32_t *>(workspace);
+    uint32_t *ka = count + 4 * table, *va = ka + n, *kb = va + n, *vb = kb + n;
+    if (cudaMemsetAsync(count + table, 0, (size_t)3 * table * 4, st) != cudaSuccess)
+        return check_launch("mi3_rank_average: memset");
+    k_rank_count<<<nb, RK_THREADS, 0, st>>>(x, n, count);
+    k_rank_pass<true><<<nb, RK_THREADS, 0, st>>>(x, nullptr, nullptr, n, 0, count, count + table, ka, va);
+    k_rank_pass<false><<<nb, RK_THREADS, 0, st>>>(nullptr, ka, va, n, 8, count + table, count + 2 * table, kb, vb);
+    k_rank_pass<false><<<nb, RK_THREADS, 0, st>>>(nullptr, kb, vb, n, 16, count + 2 * table, count + 3 * table, ka, va);
+    k_rank_pass<false><<<nb, RK_THREADS, 0, st>>>(nullptr, ka, va, n, 24, count + 3 * table, nullptr, kb, vb);
+    k_rank_scatter<<<(n + 255) / 256, 256, 0, st>>>(kb, vb, n, ranks);
     return check_launch("mi3_rank_average");
 }
 
