@@ -132,12 +132,15 @@ __device__ __forceinline__ void pair_decode_fast(uint32_t p, uint32_t L, uint32_
     j = (uint32_t)(r + 1 + ((int64_t)p - start(r)));
 }
 
-// k_gauge_apply with one warp per pair, 8 pairs per CTA.
+// k_gauge_apply with one warp per pair, 8 pairs per CTA; the pair's means and
+// fields wait in shared memory (read per element from L1 they cost more than
+// the couplings' own traffic).
 __global__ void __launch_bounds__(256) k_gauge_apply_w(const float *J, float *Jout, const double *__restrict__ m1,
                                                        const double *__restrict__ m2, const double *__restrict__ mJ,
                                                        const double *__restrict__ hd, uint32_t L, uint32_t q,
                                                        uint32_t np) {
-    const uint32_t p = blockIdx.x * 8 + (threadIdx.x >> 5), l = threadIdx.x & 31;
+    __shared__ double rows[8][4][32];
+    const uint32_t w = threadIdx.x >> 5, p = blockIdx.x * 8 + w, l = threadIdx.x & 31;
     if (p >= np) return;
     uint32_t i, j;
     pair_decode_fast(p, L, i, j);
@@ -145,11 +148,26 @@ __global__ void __launch_bounds__(256) k_gauge_apply_w(const float *J, float *Jo
     const float *Jp = J + (size_t)p * qq;
     float *Op = Jout + (size_t)p * qq;
     const double mj = mJ[p];
+    if (l < q) {
+        rows[w][0][l] = m1[(size_t)p * q + l];
+        rows[w][1][l] = m2[(size_t)p * q + l];
+        rows[w][2][l] = hd[(size_t)i * q + l];
+        rows[w][3][l] = hd[(size_t)j * q + l];
+    }
+    __syncwarp();
+    const uint32_t da = 32 / q, db = 32 - da * q;
+    uint32_t a = l / q, b = l - a * q;
+#pragma unroll 4
     for (uint32_t e = l; e < qq; e += 32) {
-        const uint32_t a = e / q, b = e - a * q;
-        double v = (double)Jp[e] - m1[(size_t)p * q + b] - m2[(size_t)p * q + a] + mj;
-        v = v + hd[(size_t)i * q + a] + hd[(size_t)j * q + b];
+        double v = (double)Jp[e] - rows[w][0][b] - rows[w][1][a] + mj;
+        v = v + rows[w][2][a] + rows[w][3][b];
         Op[e] = (float)v;
+        a += da;
+        b += db;
+        if (b >= q) {
+            b -= q;
+            ++a;
+        }
     }
 }
 
@@ -253,51 +271,73 @@ __global__ void __launch_bounds__(STAT_THREADS) k_pair_stats(const float *__rest
     }
 }
 
-// The same, one warp per pair and 8 pairs per CTA (q <= 32): lanes hold the
-// row and column sums (same order), elements e = lane + 32 k, then a
-// shuffle tree per statistic.
+// The same, one warp per pair (q <= 32): lanes hold the row and column sums
+// (same order), elements e = lane + 32 k.  Each warp takes every (8 * CTAs)-th
+// pair, then a shuffle tree per statistic and a fixed-order sum over the CTA's
+// warps: one set of partials per CTA (at most STAT_CTAS), so that the last
+// reduction reads 57 KB and not 6 MB (L=512).  Entries above the threshold are
+// queued and divided 32 at a time: nearly every group of 32 entries has one.
+constexpr uint32_t STAT_CTAS = 148 * 8;
+
 __global__ void __launch_bounds__(256) k_pair_stats_w(const float *__restrict__ tgt, const float *__restrict__ mdl,
                                                       const float *__restrict__ J, double *part, uint32_t q,
                                                       uint32_t np) {
     __shared__ double sums[8][4][32];
-    extern __shared__ float stage[];  // [8 warps][2][q q]: the pair's target and model
-    const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const uint32_t p = blockIdx.x * 8 + w;
-    if (p >= np) return;  // the whole warp
-    const uint32_t qq = q * q;
-    const float *Tg = tgt + (size_t)p * qq, *Mg = mdl + (size_t)p * qq;
+    __shared__ double red[8][NSTAT];
+    extern __shared__ float stage[];  // [8 warps][2][q q]: the pair's target and model; then [8][q q] u16 queues
+    const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31, qq = q * q;
     float *T = stage + (size_t)w * 2 * qq, *M = T + qq;
-    for (uint32_t e = l; e < qq; e += 32) {  // coalesced, all in flight
-        T[e] = Tg[e];
-        M[e] = Mg[e];
-    }
-    __syncwarp();
+    uint16_t *top = reinterpret_cast<uint16_t *>(stage + (size_t)16 * qq) + w * qq;
     double *ma = sums[w][0], *mb = sums[w][1], *ta = sums[w][2], *tb = sums[w][3];
-    if (J && l < q) {
-        double sm_r = 0, sm_c = 0, st_r = 0, st_c = 0;
-        for (uint32_t k = 0; k < q; ++k) {
-            sm_r += M[l * q + k];
-            sm_c += M[k * q + l];
-            st_r += T[l * q + k];
-            st_c += T[k * q + l];
-        }
-        ma[l] = sm_r; mb[l] = sm_c; ta[l] = st_r; tb[l] = st_c;
-    }
-    __syncwarp();
+    const uint32_t da = 32 / q, db = 32 - da * q;
     double v[NSTAT] = {0, 0, 0, 0, 0, 0};
-    for (uint32_t e = l; e < qq; e += 32) {
-        const double t = T[e], m = M[e], d = t - m;
-        v[0] += d * d;
-        v[1] = fmax(v[1], fabs(d));
-        if (T[e] > 0.01f) {
-            v[2] += fabs(d) / t;
-            v[3] += 1.0;
+    for (uint32_t p = blockIdx.x * 8 + w; p < np; p += gridDim.x * 8) {
+        const float *Tg = tgt + (size_t)p * qq, *Mg = mdl + (size_t)p * qq;
+        __syncwarp();
+        for (uint32_t e = l; e < qq; e += 32) {  // coalesced, all in flight
+            T[e] = Tg[e];
+            M[e] = Mg[e];
         }
-        if (J) {
-            const uint32_t a = e / q, b = e - a * q;
-            const double jv = J[(size_t)p * qq + e];
-            v[4] += jv * (m - ma[a] * mb[b]);
-            v[5] += jv * (t - ta[a] * tb[b]);
+        __syncwarp();
+        if (J && l < q) {
+            double sm_r = 0, sm_c = 0, st_r = 0, st_c = 0;
+            for (uint32_t k = 0; k < q; ++k) {
+                sm_r += M[l * q + k];
+                sm_c += M[k * q + l];
+                st_r += T[l * q + k];
+                st_c += T[k * q + l];
+            }
+            ma[l] = sm_r; mb[l] = sm_c; ta[l] = st_r; tb[l] = st_c;
+        }
+        __syncwarp();
+        uint32_t ntop = 0, a = l / q, b = l - a * q;
+        for (uint32_t e0 = 0; e0 < qq; e0 += 32) {
+            const uint32_t e = e0 + l;
+            const bool in = e < qq;
+            const double t = in ? T[e] : 0.0f, m = in ? M[e] : 0.0f, d = t - m;
+            v[0] += d * d;
+            v[1] = fmax(v[1], fabs(d));
+            const bool big = in && T[e] > 0.01f;
+            const uint32_t mask = __ballot_sync(0xffffffffu, big);
+            if (big) top[ntop + __popc(mask & ((1u << l) - 1u))] = (uint16_t)e;
+            ntop += __popc(mask);
+            if (J && in) {
+                const double jv = J[(size_t)p * qq + e];
+                v[4] += jv * (m - ma[a] * mb[b]);
+                v[5] += jv * (t - ta[a] * tb[b]);
+            }
+            a += da;
+            b += db;
+            if (b >= q) {
+                b -= q;
+                ++a;
+            }
+        }
+        __syncwarp();
+        for (uint32_t k = l; k < ntop; k += 32) {
+            const double t = T[top[k]], m = M[top[k]];
+            v[2] += fabs(t - m) / t;
+            v[3] += 1.0;
         }
     }
 #pragma unroll
@@ -309,13 +349,19 @@ __global__ void __launch_bounds__(256) k_pair_stats_w(const float *__restrict__ 
         }
     }
     if (l == 0) {
-        double *o = part + (size_t)p * NSTAT;
 #pragma unroll
-        for (int k = 0; k < NSTAT; ++k) o[k] = v[k];
+        for (int k = 0; k < NSTAT; ++k) red[w][k] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < NSTAT) {
+        const uint32_t k = threadIdx.x;
+        double s = red[0][k];
+        for (uint32_t x = 1; x < 8; ++x) s = k == 1 ? fmax(s, red[x][k]) : s + red[x][k];
+        part[(size_t)blockIdx.x * NSTAT + k] = s;
     }
 }
 
-// One CTA: fixed strided assignment of pairs to threads, then a fixed tree.
+// One CTA: fixed strided assignment of partials to threads, then a fixed tree.
 __global__ void __launch_bounds__(1024) k_stats_final(const double *__restrict__ part, uint32_t npairs,
                                                       double *out) {
     __shared__ double red[32];
@@ -403,15 +449,17 @@ extern "C" int mi3_bimarg_stats(const float *target, const float *model, const f
     if (np > 0x7fffffffull) return fail(MI3_ERR_ARG, "mi3_bimarg_stats: L too large");
     cudaStream_t st = as_stream(stream);
     double *part = reinterpret_cast<double *>(workspace);
+    uint32_t nparts = (uint32_t)np;
     if (q <= 32) {
-        const size_t sm = (size_t)8 * 2 * q * q * sizeof(float);
-        if (sm > 40 * 1024) cudaFuncSetAttribute(k_pair_stats_w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_pair_stats_w<<<(uint32_t)((np + 7) / 8), 256, sm, st>>>(target, model, J, part, q, (uint32_t)np);
+        const size_t sm = (size_t)8 * q * q * (2 * sizeof(float) + sizeof(uint16_t));
+        if (sm > 36 * 1024) cudaFuncSetAttribute(k_pair_stats_w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        nparts = std::min<uint32_t>((uint32_t)((np + 7) / 8), STAT_CTAS);
+        k_pair_stats_w<<<nparts, 256, sm, st>>>(target, model, J, part, q, (uint32_t)np);
     }
     else
         k_pair_stats<<<(uint32_t)np, STAT_THREADS, 4 * q * sizeof(double), st>>>(target, model, J, part, q);
     int rc = check_launch("mi3_bimarg_stats: pairs");
     if (rc) return rc;
-    k_stats_final<<<1, 1024, 0, st>>>(part, (uint32_t)np, out);
+    k_stats_final<<<1, 1024, 0, st>>>(part, nparts, out);
     return check_launch("mi3_bimarg_stats: final");
 }
