@@ -108,8 +108,8 @@ __device__ __forceinline__ void add_f32x2(unsigned long long &acc, float lo, flo
     asm("{\n\t.reg .b64 v;\n\tmov.b64 v, {%1, %2};\n\tadd.rn.f32x2 %0, %0, v;\n\t}" : "+l"(acc) : "f"(lo), "f"(hi));
 }
 
-// One sequence's B*B terms, lanes over pairs: B float partial sums (one per
-// joint row, B terms each; two rows share a packed add), added in double.
+// One sequence's B*B terms, lanes over pairs: float partial sums of 16 terms
+// (a joint row of 16, or two of 8; two rows share a packed add), added in double.
 template <int B>
 __device__ __forceinline__ double lane_energy(uint32_t jbase, const uint32_t (&row)[B], const uint32_t (&col)[B]) {
     unsigned long long part[B / 2];
@@ -129,8 +129,13 @@ __device__ __forceinline__ double lane_energy(uint32_t jbase, const uint32_t (&r
     double e = 0.0;
 #pragma unroll
     for (int th = 0; th < B / 2; ++th) {
-        e += (double)__uint_as_float((uint32_t)part[th]);
-        e += (double)__uint_as_float((uint32_t)(part[th] >> 32));
+        const float lo = __uint_as_float((uint32_t)part[th]), hi = __uint_as_float((uint32_t)(part[th] >> 32));
+        if constexpr (B == 8) {
+            e += (double)(lo + hi);
+        } else {
+            e += (double)lo;
+            e += (double)hi;
+        }
     }
     return e;
 }
@@ -154,14 +159,10 @@ __global__ void __launch_bounds__(T, 1024 / T) k_energies_joint(const float *__r
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = T / 32;
 
     if constexpr (GI * GJ == 1) {
-        // lane l stages cell c0 + l % 8 of pair p0 + l / 8 (global reads of 8
-        // consecutive cells of 4 pairs)
-        const uint32_t cgroups = (qq + 7) / 8;
-        for (uint32_t t = warp; t < cgroups * (P / 4); t += nwarps) {
-            const uint32_t c = (t % cgroups) * 8 + (lane & 7), p = (t / cgroups) * 4 + (lane >> 3);
+        slice_transpose<P, T, true>(js, qq, [&](uint32_t c, uint32_t p) {
             const uint32_t i = i0 + p / B, j = j0 + p % B;
-            if (c < qq) js[c * P + p] = (i < j && j < L) ? __ldg(&J[pair_index(i, j, L) * qq + c]) : 0.0f;
-        }
+            return (i < j && j < L) ? __ldg(&J[pair_index(i, j, L) * qq + c]) : 0.0f;
+        });
     } else {
         float *raw = js + joint_table(q, B, GI, GJ);
         const uint32_t S = joint_stage_pair(q, GJ), R = joint_stage_row(q, B, GJ);

@@ -187,6 +187,53 @@ __device__ __forceinline__ void joint_sequences(const uint32_t *__restrict__ seq
     }
 }
 
+// o[k] = v[(k + r) mod 8], r < 8 a run-time value: three conditional swaps.
+template <typename V>
+__device__ __forceinline__ void rotate8(V (&v)[8], uint32_t r) {
+#pragma unroll
+    for (uint32_t s = 1; s < 8; s <<= 1) {
+        V o[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) o[k] = (r & s) ? v[(k + s) & 7] : v[k];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) v[k] = o[k];
+    }
+}
+
+// Moves a 1 x 1 slice between its [cell][P] table in shared memory and the
+// packed [pair][cell] arrays.  A warp takes 8 cells of 32 pairs: lane l holds
+// cell c0 + l % 8 of the pairs p0 + 4 j + l / 8, j = 0..7, which is 8 consecutive
+// cells of 4 pairs per global access.  In the table those lanes would share a
+// bank per pair, eight to one; in step k lane l instead moves pair group
+// (k + l) mod 8, all 32 banks.  fn(cell, pair) gives the element to store, or
+// fn(cell, pair, v) takes the one read.
+template <uint32_t P, uint32_t T, bool TO_TABLE, typename V, typename F>
+__device__ __forceinline__ void slice_transpose(V *table, uint32_t qq, F &&fn) {
+    const uint32_t lane = threadIdx.x & 31, cl = lane & 7, pl = lane >> 3;
+    const uint32_t cgroups = (qq + 7) / 8;
+    for (uint32_t t = threadIdx.x >> 5; t < cgroups * (P / 32); t += T / 32) {
+        const uint32_t c = (t % cgroups) * 8 + cl, p0 = (t / cgroups) * 32;
+        V v[8];
+        if constexpr (TO_TABLE) {
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) v[j] = c < qq ? fn(c, p0 + 4 * j + pl) : V(0);
+            rotate8(v, cl);
+            if (c < qq) {
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) table[c * P + p0 + 4 * ((k + cl) & 7) + pl] = v[k];
+            }
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) v[k] = c < qq ? table[c * P + p0 + 4 * ((k + cl) & 7) + pl] : V(0);
+            rotate8(v, (8 - cl) & 7);
+            if (c < qq) {
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) fn(c, p0 + 4 * j + pl, v[j]);
+            }
+        }
+    }
+}
+
 // Tile configuration of an alphabet: B joint sites per block, GI x GJ sites
 // per joint pair, T threads (1024 resident threads per SM at 64 registers,
 // so T = 1024 where one table fills the SM), and the alphabet QC where joint

@@ -176,14 +176,10 @@ __global__ void __launch_bounds__(T, 1024 / T) k_pairhist_joint(const uint32_t *
         }
     };
     if constexpr (GI * GJ == 1) {
-        // lane l takes cell c0 + l % 8 of pair p0 + l / 8 -- global writes of
-        // 8 consecutive cells of 4 pairs
-        const uint32_t cgroups = (qq + 7) / 8;
-        for (uint32_t t = warp; t < cgroups * (P / 4); t += nwarps) {
-            const uint32_t c = (t % cgroups) * 8 + (lane & 7), p = (t / cgroups) * 4 + (lane >> 3);
+        slice_transpose<P, T, false>(h, qq, [&](uint32_t c, uint32_t p, uint32_t v) {
             const uint32_t i = i0 + p / B, j = j0 + p % B;
-            if (c < qq && i < j && j < L) flush(pair_index(i, j, L) * qq + c, h[c * P + p]);
-        }
+            if (i < j && j < L) flush(pair_index(i, j, L) * qq + c, v);
+        });
     } else {
         uint32_t *raw = h + joint_table(q, B, GI, GJ);
         const uint32_t S = joint_stage_pair(q, GJ), R = joint_stage_row(q, B, GJ);
@@ -618,9 +614,21 @@ static int dispatch_pairhist(const uint32_t *seq, uint32_t buflen, uint32_t nseq
     return fail(MI3_ERR_ARG, "pair histogram: q too large");
 }
 
-__global__ void k_bicounts_to_bimarg(const uint32_t *__restrict__ c, float *bi, float nseq, uint64_t n) {
-    uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) bi[k] = ((float)c[k]) / nseq;
+// Four entries a thread where the pointers are 16-byte aligned (vec), one
+// otherwise.
+__global__ void k_bicounts_to_bimarg(const uint32_t *__restrict__ c, float *bi, float nseq, uint64_t n, bool vec) {
+    const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (!vec) {
+        if (k < n) bi[k] = ((float)c[k]) / nseq;
+        return;
+    }
+    if (4 * k + 3 < n) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(c) + k);
+        reinterpret_cast<float4 *>(bi)[k] =
+            make_float4((float)v.x / nseq, (float)v.y / nseq, (float)v.z / nseq, (float)v.w / nseq);
+    } else {
+        for (uint64_t e = 4 * k; e < n; ++e) bi[e] = ((float)c[e]) / nseq;
+    }
 }
 
 // One warp per pair; the q*q row sum follows the reference's odd-aware tree
@@ -738,8 +746,10 @@ extern "C" int mi3_bicounts_to_bimarg(const uint32_t *bicount, float *bimarg, ui
     if (!bicount || !bimarg) return fail(MI3_ERR_ARG, "mi3_bicounts_to_bimarg: null pointer");
     if (L < 2 || q < 1) return fail(MI3_ERR_ARG, "mi3_bicounts_to_bimarg: bad L/q");
     uint64_t n = npairs_of(L) * q * q;
-    k_bicounts_to_bimarg<<<(uint32_t)((n + 255) / 256), 256, 0, as_stream(stream)>>>(bicount, bimarg,
-                                                                                    (float)nseq, n);
+    const bool vec = aligned(bicount, 16) && aligned(bimarg, 16);
+    const uint64_t threads = vec ? (n + 3) / 4 : n;
+    k_bicounts_to_bimarg<<<(uint32_t)((threads + 255) / 256), 256, 0, as_stream(stream)>>>(bicount, bimarg,
+                                                                                          (float)nseq, n, vec);
     return check_launch("mi3_bicounts_to_bimarg");
 }
 
