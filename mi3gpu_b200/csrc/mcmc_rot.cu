@@ -71,7 +71,7 @@
 // second of 2048-step-like calls, before (the faster of the two older kernels)
 // and now: L=48 q=4 2^14 1.4e10, 1.8e10; L=93 q=4 2^18 2.4e10, 6.0e10; L=187 q=8
 // 50688 1.0e10, 1.8e10; L=232 q=21 2^20 8.7e9, 1.16e10; L=512 q=21 2^18 3.2e9,
-// 3.47e9 (the fill: 0.9 MB of couplings per step for 384 walkers).
+// 3.7e9 (the fill: 0.9 MB of couplings per step for 448 walkers).
 #include <algorithm>
 
 #include "common.cuh"
@@ -446,15 +446,16 @@ __device__ __forceinline__ uint32_t rot_word(const uint32_t (&sq)[Y::NW], uint32
     }
 }
 
-template <typename Y, uint32_t B>
+// Word wi takes (SET) or grows by (else) `word`.
+template <typename Y, bool SET, uint32_t B>
 __device__ __forceinline__ void rot_put(uint32_t (&sq)[Y::NW], uint32_t k, uint32_t wi, uint32_t word) {
     if constexpr (B < Y::HC) {
         if (k == B) {
 #pragma unroll
             for (uint32_t w = Y::STEPS * B / Y::FPW; w <= (Y::STEPS * B + Y::STEPS - 1) / Y::FPW && w < Y::NW; ++w)
-                sq[w] = rot_sel(wi, w, word, sq[w]);
+                sq[w] = SET ? rot_sel(wi, w, word, sq[w]) : sq[w] + rot_sel(wi, w, word, 0u);
         } else {
-            rot_put<Y, B + 1>(sq, k, wi, word);
+            rot_put<Y, SET, B + 1>(sq, k, wi, word);
         }
     }
 }
@@ -486,6 +487,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_metropolis_rot(const RotParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     using Y = RotLay<BITS, NW, S>;
     constexpr uint32_t G = MODE == ROT_PAIR1 ? 1 : 2;
+    // the long rows' kernels have no register to keep the bound and the place
+    // of the residue through the chunks: they read and work them out after
+    // (L=512, 28 warps: 9.94 -> 9.47 ms per 128 steps of 2^18; the same costs
+    // L=93, q=4 2.6%)
+    constexpr bool LATE = NW > 40 && NW < 64;
     constexpr uint32_t STR = NW + 1;  // staging words per lane (odd: few bank conflicts)
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, v = lane & (Y::STEPS - 1);
     const uint32_t warps = blockDim.x >> 5;
@@ -586,7 +592,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_metropolis_rot(const RotParams p) {
             unit = second ? p.q : 1u;
         }
         const float *brow = p.bound + (size_t)pos * (p.q + 1);
-        const float bound = __ldg(&brow[mut]) + __ldg(&brow[cur]), delta = __ldg(&brow[p.q]);
+        float bound = 0.0f, delta = 0.0f;
+        if constexpr (!LATE) {
+            bound = __ldg(&brow[mut]) + __ldg(&brow[cur]);
+            delta = __ldg(&brow[p.q]);
+        }
         uint32_t offA, offB = 0;
         if constexpr (MODE == ROT_DIFF2) {
             offA = (mut * p.q + cur) * p.Q * 128;
@@ -599,6 +609,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_metropolis_rot(const RotParams p) {
         if constexpr (S > 1) sum += __shfl_xor_sync(0xffffffffu, sum, 16);
         if constexpr (S > 2) sum += __shfl_xor_sync(0xffffffffu, sum, 8);
 
+        if constexpr (LATE) {
+            bound = __ldg(&brow[mut]) + __ldg(&brow[cur]);
+            delta = __ldg(&brow[p.q]);
+        }
         const float dE = (float)(int32_t)sum * delta;
         const float u = uniform_map(r1);
         const float x = -Bta * dE;
@@ -651,8 +665,14 @@ __global__ void __launch_bounds__(MAXT, 1) k_metropolis_rot(const RotParams p) {
             if (v == vv) acc = accept_exp(-Bta * ref, u);
             __syncwarp();
         }
-        const uint32_t moved = word + ((mut - cur) * unit << o.sh);
-        rot_put<Y, 0>(sq, o.k, acc && o.owner == lane ? o.wi : 0xffffffffu, moved);
+        if constexpr (LATE) {
+            const RotPlace o2 = rot_place<Y>(pos / G, v, p.nc, p.tail);
+            const uint32_t step = (mut - cur) * (G == 2 && (pos & 1) ? p.q : 1u) << o2.sh;
+            rot_put<Y, false, 0>(sq, o2.k, acc && o2.owner == lane ? o2.wi : 0xffffffffu, step);
+        } else {
+            const uint32_t moved = word + ((mut - cur) * unit << o.sh);
+            rot_put<Y, true, 0>(sq, o.k, acc && o.owner == lane ? o.wi : 0xffffffffu, moved);
+        }
     }
 
     // ---- every copy started must land before the ring is reused
@@ -699,7 +719,7 @@ struct RotPick {
 // leave 64, 72, 80 or 128 each; the loop needs about 30 beside the words.
 template <int MODE, uint32_t BITS, uint32_t NW, uint32_t S>
 static RotPick rot_pick() {
-    constexpr uint32_t MAXT = NW <= 28 ? 1024 : NW <= 40 ? 896 : NW <= 48 ? 768 : 512;
+    constexpr uint32_t MAXT = NW <= 28 ? 1024 : NW <= 43 ? 896 : NW <= 48 ? 768 : 512;
     return RotPick{k_metropolis_rot<MODE, BITS, NW, S, MAXT>, BITS, NW, S, MAXT};
 }
 

@@ -482,7 +482,7 @@ class MCMCGPU:
     # The rotated sampler (mi3_metropolis_rot) gives the same trajectories and
     # is the fastest where it applies (B200, site-updates/s against the best
     # of the other two: L=93 q=4 2^18 6.0e10 / 2.4e10, L=232 q=21 2^20 1.16e10
-    # / 8.7e9, L=512 q=21 2^18 3.5e9 / 3.2e9).  sampler_rot: None uses it unless a plan was
+    # / 8.7e9, L=512 q=21 2^18 3.7e9 / 3.2e9).  sampler_rot: None uses it unless a plan was
     # installed as metro_plan, True / False (set by autotune.Autotuner.tune from
     # its timings) decides.
     sampler_rot = None
