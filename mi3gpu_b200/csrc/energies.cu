@@ -287,16 +287,19 @@ template <bool CONS>
 static int dispatch_energies(const float *J, const uint32_t *seq, uint32_t buflen, uint32_t nseq,
                              unsigned long long *acc, uint32_t L, uint32_t q, const uint8_t *cons,
                              cudaStream_t st) {
+    // Sequences of a few sites take the pair-major kernel whatever the alphabet:
+    // among them many walkers are equal or have energies a last bit apart, and
+    // the rank transform of the equilibration test would turn sums rounded in
+    // another order into other ranks.  (Their passes take microseconds.)
+    const bool few_sites = L < (q <= 10 ? 32u : 16u);
     if constexpr (!CONS) {
         int rc = MI3_OK;
-        if (joint_dispatch(q, [&](auto cfg) { rc = launch_energies_joint<decltype(cfg)>(J, seq, buflen, nseq, acc, L, q, st); }))
+        if (!few_sites && joint_dispatch(q, [&](auto cfg) { rc = launch_energies_joint<decltype(cfg)>(J, seq, buflen, nseq, acc, L, q, st); }))
             return rc;
     }
     const uint32_t B = pick_block(q, 116 * 1024, 16);
-    if constexpr (CONS) {
-        if (B == 16) return launch_energies<16, true>(J, seq, buflen, nseq, acc, L, q, cons, st);
-        if (B == 8) return launch_energies<8, true>(J, seq, buflen, nseq, acc, L, q, cons, st);
-    }
+    if (B == 16) return launch_energies<16, CONS>(J, seq, buflen, nseq, acc, L, q, cons, st);
+    if (B == 8) return launch_energies<8, CONS>(J, seq, buflen, nseq, acc, L, q, cons, st);
     if (B == 4) return launch_energies<4, CONS>(J, seq, buflen, nseq, acc, L, q, cons, st);
     return fail(MI3_ERR_ARG, "mi3_energies: q too large");
 }
