@@ -769,9 +769,13 @@ static size_t rot_smem(const RotShape &r, const RotPick &k, uint32_t warps, uint
     return ROT_HEAD + (((size_t)warps * k.S * k.nw * 4 + 127) & ~size_t(127)) + std::max(ring, staging);
 }
 
-// Two steps' chunks ahead (at least 3 slots, at most 6) where they fit.
+// Two steps' chunks ahead (at least 3 slots, at most 6) where they fit.  CTAs of
+// few warps wait rather than compute and take two slots, so that CTAs of
+// problems on other streams fit beside them: L=100, 8192 walkers, three problems
+// in turn, q=4 243 -> 134 us each, q=21 526 -> 326, alone 358 -> 349 and 666 -> 651.
 static uint32_t rot_slots(const RotShape &r, const RotPick &k, uint32_t warps) {
-    for (uint32_t s = std::max(3u, std::min(2 * r.nc, ROT_MAX_SLOTS)); s >= 2; --s)
+    const uint32_t most = warps <= 8 ? 2 : std::max(3u, std::min(2 * r.nc, ROT_MAX_SLOTS));
+    for (uint32_t s = most; s >= 2; --s)
         if (rot_smem(r, k, warps, s) <= 227 * 1024) return s;
     return 0;
 }
@@ -847,8 +851,19 @@ extern "C" int mi3_metropolis_rot(const float *Jrot, uint32_t *rngstates, uint32
         return fail(MI3_ERR_ARG, "mi3_metropolis_rot: nseqs must be a positive multiple of 32");
     if (!aligned(Jrot, 16) || !aligned(rngstates, 16))
         return fail(MI3_ERR_ALIGN, "mi3_metropolis_rot: Jrot/rngstates must be 16B aligned");
-    uint32_t warps = 0;
-    const RotPick k = rot_plan(r, nseqs, walkers_per_cta, lanes_per_walker, warps);
+    // the plan of the thread's last call, while the call has the same sizes
+    static thread_local struct {
+        uint32_t L = 0, q, nseqs, walkers, lanes, warps;
+        RotPick k;
+    } last;
+    if (last.L != L || last.q != q || last.nseqs != nseqs || last.walkers != walkers_per_cta ||
+        last.lanes != lanes_per_walker) {
+        last.warps = 0;
+        last.k = rot_plan(r, nseqs, walkers_per_cta, lanes_per_walker, last.warps);
+        last.L = L, last.q = q, last.nseqs = nseqs, last.walkers = walkers_per_cta, last.lanes = lanes_per_walker;
+    }
+    const uint32_t warps = last.warps;
+    const RotPick k = last.k;
     if (!k.kernel)
         return fail(MI3_ERR_ARG, "mi3_metropolis_rot: no kernel with these walkers per CTA and lanes per walker");
     if (nsteps == 0) return MI3_OK;

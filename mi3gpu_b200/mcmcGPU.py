@@ -464,8 +464,8 @@ class MCMCGPU:
     # ------------------------------------------------------------ sampler plans
     # The skewed-lane sampler (mi3_metropolis_skew) gives the same
     # trajectories as the row-streaming one; it takes q <= 21 and
-    # L + 31 <= 288.  Untuned, it is used from SKEW_MIN_Q on with at least
-    # one CTA per SM (B200, 2048-step calls: 8.7e9 vs 6.1e9 site-updates/s at
+    # L + 31 <= 576.  Untuned, and where sampler_kernel() leaves the plan to
+    # choose, it is used from SKEW_MIN_Q on with at least one CTA per SM (B200, 2048-step calls: 8.7e9 vs 6.1e9 site-updates/s at
     # L=232, q=21, 2^20 walkers; even at L=60, q=21; slower at q=4, where
     # the row kernel's gathers mostly hit the same address and broadcast).
     SKEW_DEFAULT = True
@@ -479,23 +479,34 @@ class MCMCGPU:
         (L + 31 <= 288 with 512 or 768 walkers per CTA, else 256)."""
         return 2 <= self.q <= 21 and self.L + 31 <= 576 and self.nseq['main'] % 32 == 0
 
-    # The rotated sampler (mi3_metropolis_rot) gives the same trajectories and
-    # is the fastest where it applies (B200, site-updates/s against the best
-    # of the other two: L=93 q=4 2^18 6.0e10 / 2.4e10, L=232 q=21 2^20 1.16e10
-    # / 8.7e9, L=512 q=21 2^18 3.7e9 / 3.2e9).  sampler_rot: None uses it unless a plan was
-    # installed as metro_plan, True / False (set by autotune.Autotuner.tune from
-    # its timings) decides.
+    # The rotated sampler (mi3_metropolis_rot) gives the same trajectories
+    # (B200, site-updates/s against the best of the other two: L=93 q=4 2^18
+    # 6.0e10 / 2.4e10, L=232 q=21 2^20 1.16e10 / 8.7e9, L=512 q=21 2^18 3.7e9 /
+    # 3.2e9).  sampler_rot: None uses it by the rule of rot_default unless a
+    # plan was installed as metro_plan, True / False (set by
+    # autotune.Autotuner.tune from its timings) decides.
     sampler_rot = None
 
     def rot_supported(self):
         return 2 <= self.q <= 21 and 2 <= self.L <= 576 and self.nseq['main'] % 32 == 0
+
+    def rot_default(self):
+        """Where the rotated sampler is used untuned.  With few walkers its
+        CTAs are a few warps that wait for their row's copies, and its rows
+        are the longer the larger q: three problems in turn on three streams,
+        2 L proposals after new couplings, time of the older kernels over its
+        own (in brackets one problem alone): L=100 q=4 8192 walkers 1.13
+        (1.18), 49152 1.21 (1.74); q=8 16384 0.61 (1.03), 49152 1.04 (1.51);
+        q=21 8192 0.81 (1.04), 49152 1.16 (1.62); L=37 q=8 49152 0.80 (1.12),
+        L=37 q=4 8192 0.93 (1.02), L=48 q=4 16384 1.14 (1.04)."""
+        return self.L >= (48 if self.q <= 5 else 64) and (self.q <= 5 or self.nseq['main'] >= 49152)
 
     def sampler_kernel(self):
         """The sampler runMCMC runs: 'rot' (mi3_metropolis_rot) or 'plan' (the
         kernel and tiles of sampler_plan())."""
         want = self.sampler_rot
         if want is None:
-            want = not getattr(self, 'metro_plan', None)
+            want = not getattr(self, 'metro_plan', None) and self.rot_default()
         return 'rot' if want and self.rot_supported() else 'plan'
 
     def sampler_plan(self):

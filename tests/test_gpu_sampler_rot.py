@@ -120,3 +120,23 @@ def test_rot_bad_site_reported_and_shapes_refused(cuda):
         with pytest.raises(_lib.Mi3Error):
             _lib.call("mi3_metropolis_rot", buf.data_ptr(), buf.data_ptr(), 0, buf.data_ptr(), 1, None, 1.0,
                       buf.data_ptr(), N, L, q, wpc, lanes, status.data_ptr(), stream())
+
+
+@pytest.mark.parametrize("L,q,kind", [(47, 4, "plan"), (48, 4, "rot"), (64, 6, "plan")])
+def test_untuned_choice_keeps_the_trajectories(cuda, L, q, kind):
+    """Both sides of rot_default: the same walkers and generators as with the
+    other kernel, bit for bit."""
+    from mi3gpu_b200.mcmcGPU import MCMCGPU
+    N, out = 512, []
+    for rot in (None, kind == "plan"):
+        g = MCMCGPU((0, 0), L, q, N, 512, None, 1024, 3)
+        assert g.sampler_kernel() == kind
+        g.initMCMC(100)
+        g.setBuf("J", random_model(L, q, 4))
+        g.setBuf("seq main", oracle.pack_seqs(_seqs(L, q, N, 5)))
+        g.sampler_rot = rot
+        g.runMCMC()
+        out.append((g.getBuf("seq main").read(), g.getBuf("rngstates").read()))
+        g.wait()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
