@@ -133,7 +133,7 @@ def test_untuned_choice_keeps_the_trajectories(cuda, L, q, kind):
         assert g.sampler_kernel() == kind
         g.initMCMC(100)
         g.setBuf("J", random_model(L, q, 4))
-        g.setBuf("seq main", oracle.pack_seqs(_seqs(L, q, N, 5)))
+        g.setBuf("seq main", oracle.pack_seqs(np.random.default_rng(5).integers(0, q, size=(N, L)).astype("<u1")))
         g.sampler_rot = rot
         g.runMCMC()
         out.append((g.getBuf("seq main").read(), g.getBuf("rngstates").read()))
