@@ -127,11 +127,12 @@ def test_untuned_choice_keeps_the_trajectories(cuda, L, q, kind):
     """Both sides of rot_default: the same walkers and generators as with the
     other kernel, bit for bit."""
     from mi3gpu_b200.mcmcGPU import MCMCGPU
+    from mi3gpu_b200.node_manager import GPU_node
     N, out = 512, []
     for rot in (None, kind == "plan"):
         g = MCMCGPU((0, 0), L, q, N, 512, None, 1024, 3)
         assert g.sampler_kernel() == kind
-        g.initMCMC(100)
+        GPU_node([g]).initMCMC(100)
         g.setBuf("J", random_model(L, q, 4))
         g.setBuf("seq main", oracle.pack_seqs(np.random.default_rng(5).integers(0, q, size=(N, L)).astype("<u1")))
         g.sampler_rot = rot
