@@ -126,18 +126,17 @@ def test_rot_bad_site_reported_and_shapes_refused(cuda):
 def test_untuned_choice_keeps_the_trajectories(cuda, L, q, kind):
     """Both sides of rot_default: the same walkers and generators as with the
     other kernel, bit for bit."""
-    from mi3gpu_b200.mcmcGPU import MCMCGPU
-    from mi3gpu_b200.node_manager import GPU_node
+    from mi3gpu_b200 import GPU_node, MCMCGPU
     N, out = 512, []
     for rot in (None, kind == "plan"):
         g = MCMCGPU((0, 0), L, q, N, 512, None, 1024, 3)
         assert g.sampler_kernel() == kind
-        GPU_node([g]).initMCMC(100)
-        g.setBuf("J", random_model(L, q, 4))
-        g.setBuf("seq main", oracle.pack_seqs(np.random.default_rng(5).integers(0, q, size=(N, L)).astype("<u1")))
+        node = GPU_node([g])
+        node.initMCMC(100)
+        node.setSeqs("main", np.random.default_rng(5).integers(0, q, size=(N, L)).astype("<u1"))
+        node.setBuf("J", random_model(L, q, 4))
         g.sampler_rot = rot
-        g.runMCMC()
-        out.append((g.getBuf("seq main").read(), g.getBuf("rngstates").read()))
-        g.wait()
+        node.runMCMC()
+        out.append((node.collect("seq main"), g.getBuf("rngstates").read()))
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
