@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(1024) k_unpack_rot(const float *__restrict__ J
             float big = 0.0f;
             for (uint32_t s = 0; s < q; ++s) {
                 const float v = fabsf(j_at(J, L, q, pos, m, lane, s));
-                big = v <= big ? big : v;  // keeps a NaN
+                big = isnan(big) || v <= big ? big : v;  // a NaN stays, and makes the bound infinite
             }
             W += big;
             R += (fabsf((float)(L / 2) - (float)m) + 2.0f) * big;

@@ -109,6 +109,26 @@ def test_rot_infinite_and_huge_couplings(cuda, L, q):
     np.testing.assert_array_equal(g_st, o_st)
 
 
+@pytest.mark.parametrize("last", [False, True])
+@pytest.mark.parametrize("L,q", [(20, 4), (20, 8), (40, 21)])
+def test_rot_nan_couplings(cuda, L, q, last):
+    """A NaN coupling, whatever its residues, leaves the verdicts of its letters
+    to the exact sum, which rejects the moves that meet it."""
+    J = random_model(L, q, 11)
+    rng = np.random.default_rng(q)
+    cells = rng.integers(0, q - 1, size=(2, 24)) if not last else np.full((2, 24), q - 1)
+    J[rng.integers(0, J.shape[0], 24), cells[0] * q + cells[1]] = np.nan
+    N, nsteps = 512, 6 * L
+    mem, st, pos = _start(L, q, N, nsteps, 4)
+    o_mem, o_st = mem.copy(), st.copy()
+    oracle.metropolis(J, o_st, pos, 0, nsteps, o_mem, L, q)
+    for lanes in (1, 2, 4):
+        g_mem, g_st, status = _run(_table(J, L, q), mem, st, pos, nsteps, L, q, 0, lanes=lanes)
+        assert status == 0
+        np.testing.assert_array_equal(g_mem, o_mem)
+        np.testing.assert_array_equal(g_st, o_st)
+
+
 def test_rot_bad_site_reported_and_shapes_refused(cuda):
     L, q, N = 16, 4, 512
     T = _table(random_model(L, q, 6), L, q)
