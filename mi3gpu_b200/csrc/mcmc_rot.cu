@@ -622,7 +622,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_metropolis_rot(const RotParams p) {
         const float e = expf(x), tol = xb + xb * xb + 0x1p-20f;
         bool acc = e * (1.0f - tol) > fmaxf(u, 1e-30f);
         bool sure = xb <= 0.25f && (acc || e * (1.0f + tol) < u);
-        if (x >= xb) acc = sure = true;
+        // (an infinite x says nothing about dE: it may be within its bound of 0)
+        if (x >= xb && xb < __int_as_float(0x7f800000)) acc = sure = true;
         uint32_t open = __ballot_sync(0xffffffffu, !sure && valid) & (0xffffffffu >> (32 - Y::STEPS));
         while (open) {
             // the warp sums walker vv's terms in site order

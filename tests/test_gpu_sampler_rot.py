@@ -129,6 +129,23 @@ def test_rot_nan_couplings(cuda, L, q, last):
         np.testing.assert_array_equal(g_st, o_st)
 
 
+@pytest.mark.parametrize("L,q", [(20, 4), (21, 7), (40, 21)])
+def test_rot_infinite_beta(cuda, L, q):
+    """beta * dE overflows: the verdict hangs on the sign of dE.  Couplings in
+    tenths, so that many differences are 0 but for the rounding of the sum."""
+    rng = np.random.default_rng(q)
+    J = (rng.integers(0, 4, size=(L * (L - 1) // 2, q * q)) / 10).astype("<f4")
+    N, nsteps = 512, 4 * L
+    mem, st, pos = _start(L, q, N, nsteps, 6)
+    betas = np.resize(np.array([np.inf, 3e38, 1e38, -np.inf, 1.0], "<f4"), N)
+    o_mem, o_st = mem.copy(), st.copy()
+    oracle.metropolis(J, o_st, pos, 0, nsteps, o_mem, L, q, betas=betas)
+    g_mem, g_st, status = _run(_table(J, L, q), mem, st, pos, nsteps, L, q, 0, betas=betas)
+    assert status == 0
+    np.testing.assert_array_equal(g_mem, o_mem)
+    np.testing.assert_array_equal(g_st, o_st)
+
+
 def test_rot_bad_site_reported_and_shapes_refused(cuda):
     L, q, N = 16, 4, 512
     T = _table(random_model(L, q, 6), L, q)
