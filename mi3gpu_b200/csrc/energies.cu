@@ -1,16 +1,22 @@
 // energies.cu -- Potts energies E(s) = sum_{i<j} J_ij(s_i, s_j).
 //
-// Slice-tiled (tiling.cuh): a CTA holds the couplings of one block pair in
-// shared memory and streams a chunk of sequences through it; each thread
-// sums its sequence's gathered couplings (float within a site row of at most
-// B terms, double across rows) and adds the slice total to a per-sequence
-// 64-bit fixed-point accumulator (scale 2^40) with an integer atomic.
-// Integer addition is associative, so the result does not depend on CTA
-// order: energies are deterministic.  The float row sums bound the error at
-// about B*2^-24 of the largest row sum per row, far below the final
-// rounding to float for the energies the sampler meets.  The reference sums each
-// sequence serially with Kahan compensation in float (getEnergiesf,
-// mcmc.cl:249-336); this result is at least as accurate.
+// A CTA holds the couplings of one block pair (slice) in shared memory and
+// streams a chunk of sequences through it; each thread sums its sequence's
+// gathered couplings, floats first and those sums in double, and adds the slice
+// total to a per-sequence 64-bit fixed-point accumulator (scale 2^40) with an
+// integer atomic.  Integer addition is associative, so the result does not
+// depend on CTA order, and within a slice a sequence's sum has the same bits
+// whichever lane takes it: energies are functions of the residues alone, and
+// copies of a sequence tie.
+//
+// How often a coupling is rounded in float, at 2^-24 of its partial sum each:
+//   joint sites (joint.cuh, q <= 21): 0, 1 or 2 times where a cell sums 1, 2 or
+//     4 couplings, and 4 times in a tree of 16 cells -- 4 to 6 in all;
+//   pair-major (tiling.cuh: larger alphabets, few sites, the consensus gauge):
+//     up to B - 1 = 3, 7 or 15 times along its site row.
+// Both are far below the final rounding to float for the energies the sampler
+// meets.  The reference sums each sequence serially with Kahan compensation in
+// float (getEnergiesf, mcmc.cl:249-336), to about two roundings of the total.
 #include <mutex>
 
 #include "joint.cuh"
@@ -103,41 +109,47 @@ __device__ __forceinline__ void energies_chunk(const float *js, const uint32_t *
     }
 }
 
-// (hi, lo) floats += (hi, lo) floats: two independent float adds.
-__device__ __forceinline__ void add_f32x2(unsigned long long &acc, float lo, float hi) {
-    asm("{\n\t.reg .b64 v;\n\tmov.b64 v, {%1, %2};\n\tadd.rn.f32x2 %0, %0, v;\n\t}" : "+l"(acc) : "f"(lo), "f"(hi));
+// Two floats, gathered or added as a pair.
+__device__ __forceinline__ unsigned long long gather_f32x2(uint32_t lo_at, uint32_t hi_at) {
+    unsigned long long v;
+    asm volatile("{\n\t.reg .f32 lo, hi;\n\tld.shared.f32 lo, [%1];\n\tld.shared.f32 hi, [%2];\n\tmov.b64 %0, {lo, hi};\n\t}"
+                 : "=l"(v)
+                 : "r"(lo_at), "r"(hi_at));
+    return v;
+}
+__device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
 }
 
-// One sequence's B*B terms, lanes over pairs: float partial sums of 16 terms
-// (a joint row of 16, or two of 8; two rows share a packed add), added in double.
+// The cells of two rows in the N columns from step T on, N a power of two that
+// divides T: a balanced tree, so the sums are the same in every lane (tiling.cuh)
+// and a cell is rounded log2(N) times.
+template <int B, int T, int N>
+__device__ __forceinline__ unsigned long long rows_sum(const uint32_t (&col)[B], uint32_t row0, uint32_t row1) {
+    if constexpr (N == 1)
+        return gather_f32x2(col[T] + row0, col[T] + row1);
+    else
+        return add_f32x2(rows_sum<B, T, N / 2>(col, row0, row1), rows_sum<B, T + N / 2, N / 2>(col, row0, row1));
+}
+
+// One sequence's B*B terms, lanes over pairs: trees of 16 in float (a joint row
+// of 16, or two of 8), whose sums are added as a tree in double.
 template <int B>
-__device__ __forceinline__ double lane_energy(uint32_t jbase, const uint32_t (&row)[B], const uint32_t (&col)[B]) {
-    unsigned long long part[B / 2];
-#pragma unroll
-    for (int th = 0; th < B / 2; ++th) part[th] = 0;
-#pragma unroll
-    for (int tl = 0; tl < B; ++tl) {
-        const uint32_t c = jbase + col[tl];
-#pragma unroll
-        for (int th = 0; th < B / 2; ++th) {
-            float v0, v1;
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v0) : "r"(c + row[2 * th]));
-            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v1) : "r"(c + row[2 * th + 1]));
-            add_f32x2(part[th], v0, v1);
-        }
-    }
-    double e = 0.0;
+__device__ __forceinline__ double lane_energy(const uint32_t (&row)[B], const uint32_t (&col)[B]) {
+    double e[B / 2];
 #pragma unroll
     for (int th = 0; th < B / 2; ++th) {
-        const float lo = __uint_as_float((uint32_t)part[th]), hi = __uint_as_float((uint32_t)(part[th] >> 32));
-        if constexpr (B == 8) {
-            e += (double)(lo + hi);
-        } else {
-            e += (double)lo;
-            e += (double)hi;
-        }
+        const unsigned long long v = rows_sum<B, 0, B>(col, row[2 * th], row[2 * th + 1]);
+        const float lo = __uint_as_float((uint32_t)v), hi = __uint_as_float((uint32_t)(v >> 32));
+        e[th] = B == 8 ? (double)(lo + hi) : (double)lo + (double)hi;
     }
-    return e;
+#pragma unroll
+    for (int s = 1; s < B / 2; s <<= 1)
+#pragma unroll
+        for (int th = 0; th < B / 2; th += 2 * s) e[th] += e[th + s];
+    return e[0];
 }
 
 // Energies over joint sites (joint.cuh).  Bound by instruction issue at two
@@ -198,9 +210,9 @@ __global__ void __launch_bounds__(T, 1024 / T) k_energies_joint(const float *__r
 
     const uint32_t nbeg = chunk * g.chunk, nend = min(nseq, nbeg + g.chunk);
     const uint32_t jbase = (uint32_t)__cvta_generic_to_shared(js);
-    joint_sequences<B, GI, GJ>(seq, buflen, nbeg, nend, L, q, bi, bj,
+    joint_sequences<B, GI, GJ>(seq, buflen, nbeg, nend, L, q, bi, bj, jbase,
                                [&](const uint32_t(&row)[B], const uint32_t(&col)[B], uint32_t n) {
-                                   const double e = lane_energy<B>(jbase, row, col);
+                                   const double e = lane_energy<B>(row, col);
                                    atomicAdd(&acc[n], (unsigned long long)__double2ll_rn(e * FIX_SCALE));
                                });
 }
@@ -287,10 +299,12 @@ template <bool CONS>
 static int dispatch_energies(const float *J, const uint32_t *seq, uint32_t buflen, uint32_t nseq,
                              unsigned long long *acc, uint32_t L, uint32_t q, const uint8_t *cons,
                              cudaStream_t st) {
-    // Sequences of a few sites take the pair-major kernel whatever the alphabet:
-    // among them many walkers are equal or have energies a last bit apart, and
-    // the rank transform of the equilibration test would turn sums rounded in
-    // another order into other ranks.  (Their passes take microseconds.)
+    // Sequences shorter than two blocks of the pair-major tiling keep its sums.
+    // Among so few sites the walkers are groups of many equal ones, and two groups
+    // whose energies are a last bit apart trade ranks where the sums are rounded
+    // in another order, each walker by the size of the other group (L=16, q=2,
+    // 2^18 walkers: by 133 ranks).  The price is time: 194 us where the joint kernel takes 65
+    // at L=20, q=4, 2^20; 32 and 22 us at 2^14.
     const bool few_sites = L < (q <= 10 ? 32u : 16u);
     if constexpr (!CONS) {
         int rc = MI3_OK;

@@ -21,17 +21,17 @@
 // (q=5 2x2 leaves 26 KB for staging; q=6 2x2 would need 332 KB).  Larger
 // alphabets (22..42) keep the pair-major kernels of tiling.cuh.
 //
-// Tables are cell-major, [cell][P], P = B*B joint pairs, and lanes visit
-// pairs in rotated order (tiling.cuh), so every access is one wavefront.
+// Tables are cell-major, [cell][P], P = B*B joint pairs, and each lane visits
+// the pairs in its own order (tiling.cuh), so every access is one wavefront.
 // Slices that cross the diagonal or the end of the sequence run the same
 // code: their invalid site pairs add zero couplings, or are not flushed.
 //
 // Measured against the pair-major tiling with lanes over pairs in full slices
 // only (Newton phases on one B200, l1z or l2z included):
-//   L=93  q=4  2^18  8 steps   10.0 -> 2.37 ms (2.92 with the alphabet a
+//   L=93  q=4  2^18  8 steps   10.0 -> 2.23 ms (2.92 with the alphabet a
 //                              run-time value in the packing and splitting)
-//   L=151 q=8  66048 8 steps   5.55 -> 3.14 ms (3.58)
-//   L=232 q=21 2^20  3 steps   38.6 -> 36.7 ms (edge slices, packed adds, one
+//   L=151 q=8  66048 8 steps   5.55 -> 2.87 ms (3.58)
+//   L=232 q=21 2^20  3 steps   38.6 -> 35.4 ms (edge slices, packed adds, one
 //                              clamp test per word)
 #pragma once
 #include "tiling.cuh"
@@ -119,29 +119,30 @@ __device__ __forceinline__ void joint_words(const uint32_t (&w)[G * B / 4], uint
     }
 }
 
-// Per-lane constants of the rotated order: byte offsets of the lane's row and
-// column positions (k + w) mod B.  Hoisted out of the sequence loop.
+// Per-lane constants of the lane's order: shared-memory address of the table
+// (at `base`) plus row position k ^ w, and byte offset of column position
+// k ^ w.  Hoisted out of the sequence loop.
 template <int B>
 struct LaneConst {
     uint32_t row[B], col[B], wh, wl;
-    __device__ __forceinline__ explicit LaneConst(uint32_t lane) : wh(lane / B), wl(lane % B) {
+    __device__ __forceinline__ LaneConst(uint32_t lane, uint32_t base) : wh(lane / B), wl(lane % B) {
 #pragma unroll
         for (int k = 0; k < B; ++k) {
-            row[k] = 4 * B * ((k + wh) & (B - 1));
-            col[k] = 4 * ((k + wl) & (B - 1));
+            row[k] = base + 4 * B * (k ^ wh);
+            col[k] = 4 * (k ^ wl);
         }
     }
 };
 
-// Byte offsets in the [cell][P] table of the lane's row terms (joint row
-// state A: A*QJ cells) and column terms, in rotated order.
+// Addresses in the [cell][P] table of the lane's row terms (joint row state A:
+// A*QJ cells) and byte offsets of its column terms, in the lane's order.
 template <int B>
 __device__ __forceinline__ void joint_offsets(const uint32_t (&sI)[B / 4], const uint32_t (&sJ)[B / 4],
                                               uint32_t row_scale, const LaneConst<B> &lc, uint32_t (&row)[B],
                                               uint32_t (&col)[B]) {
     uint32_t rI[B / 4], rJ[B / 4];
-    rotate_block<B>(sI, lc.wh, rI);
-    rotate_block<B>(sJ, lc.wl, rJ);
+    permute_block<B>(sI, lc.wh, rI);
+    permute_block<B>(sJ, lc.wl, rJ);
 #pragma unroll
     for (int k = 0; k < B; ++k) {
         row[k] = __byte_perm(rI[k >> 2], 0, 0x4440 + (k & 3)) * row_scale + lc.row[k];
@@ -156,15 +157,15 @@ __device__ __forceinline__ void load_words(const uint32_t *__restrict__ seq, uin
     for (int k = 0; k < W; ++k) w[k] = (w0 + k < swords) ? __ldg(&seq[(size_t)(w0 + k) * buflen + n]) : 0u;
 }
 
-// fn(row offsets, column offsets, n) for every sequence of [nbeg, nend) that
+// fn(row addresses, column offsets, n) for every sequence of [nbeg, nend) that
 // this thread takes; the next sequence's words load while one is processed.
 template <int B, int GI, int GJ, typename F>
 __device__ __forceinline__ void joint_sequences(const uint32_t *__restrict__ seq, uint32_t buflen, uint32_t nbeg,
                                                 uint32_t nend, uint32_t L, uint32_t q, uint32_t bi, uint32_t bj,
-                                                F &&fn) {
+                                                uint32_t base, F &&fn) {
     constexpr int WI = GI * B / 4, WJ = GJ * B / 4;
     const uint32_t swords = (L - 1) / 4 + 1;
-    const LaneConst<B> lc(threadIdx.x & 31);
+    const LaneConst<B> lc(threadIdx.x & 31, base);
     const uint32_t row_scale = 4 * B * B * joint_states(q, GJ);
     uint32_t n = nbeg + threadIdx.x;
     if (n >= nend) return;

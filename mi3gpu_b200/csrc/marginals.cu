@@ -122,7 +122,7 @@ __device__ __forceinline__ void hist_chunk(uint32_t *h, const uint32_t *__restri
 }
 
 // Histograms over joint sites (joint.cuh): [cell][P] bins, each lane adds to
-// the pairs in its own rotated order, so the 32 lanes of a shared-memory
+// the pairs in its own order, so the 32 lanes of a shared-memory
 // reduction always hit 32 different banks and different bins (no serialised
 // same-bin adds either).  The flush splits a joint bin back into the site
 // pairs it counts; sums of a chunk's increments fit u32 (fixed_shift).  Bound by
@@ -151,17 +151,16 @@ __global__ void __launch_bounds__(T, 1024 / T) k_pairhist_joint(const uint32_t *
 
     const uint32_t nbeg = chunk * g.chunk, nend = min(nseq, nbeg + g.chunk);
     const uint32_t hbase = (uint32_t)__cvta_generic_to_shared(h);
-    joint_sequences<B, GI, GJ>(seq, buflen, nbeg, nend, L, q, bi, bj,
+    joint_sequences<B, GI, GJ>(seq, buflen, nbeg, nend, L, q, bi, bj, hbase,
                                [&](const uint32_t(&row)[B], const uint32_t(&col)[B], uint32_t n) {
                                    uint32_t inc = 1u;
                                    if constexpr (WEIGHTED) inc = __float2uint_rn(__ldg(&weights[n]) * scale);
 #pragma unroll
-                                   for (int tl = 0; tl < B; ++tl) {
-                                       const uint32_t c = hbase + col[tl];
+                                   for (int tl = 0; tl < B; ++tl)
 #pragma unroll
                                        for (int th = 0; th < B; ++th)
-                                           asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(c + row[th]), "r"(inc));
-                                   }
+                                           asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(col[tl] + row[th]),
+                                                        "r"(inc));
                                });
     __syncthreads();
 

@@ -165,33 +165,35 @@ __device__ __forceinline__ uint32_t slice_row(const uint32_t (&wI)[B / 4], int i
 // shared-memory wavefronts per warp instruction.  For q <= 21 (joint.cuh) the
 // pair kernels lay the table out cell-major instead, [cell][p] with P = B*B
 // pairs (p = ii*B + jj).  Lane w = B*wh + wl visits, at
-// step (th, tl), the pair ii = (th + wh) mod B, jj = (tl + wl) mod B.  Its bank
-// is (ii*B + jj) mod 32: the B lanes of one wh hold B different jj, and the
-// 32/B values of wh hold ii that differ mod 32/B, so the 32 lanes use 32
-// different banks at every step -- one wavefront.  Rotating the sequence's
-// residue bytes of block I by wh and of block J by wl (byte k of the rotated
-// block = byte (k + r) mod B) makes the offsets static register indices: one
-// add, row[th] + col[tl], per pair.  (Visiting pair (t + w) mod P instead
-// needs a select per pair where t + w carries into the next row, on the
-// half-rate ALU: a Newton phase of 3 steps at L=232, q=21, 2^20 -- four energy
-// passes, a count and three weighted passes -- took 44.3 ms that way, 38.6 ms
-// this way.)  B >= 8.
+// step (th, tl), the pair ii = th ^ wh, jj = tl ^ wl.  Its bank is
+// (ii*B + jj) mod 32: the B lanes of one wh hold B different jj, and the 32/B
+// values of wh hold ii that differ mod 32/B, so the 32 lanes use 32 different
+// banks at every step -- one wavefront.  Permuting the sequence's residue bytes
+// of block I by wh and of block J by wl (byte k of the permuted block = byte
+// k ^ r) makes the offsets static register indices: one add, row[th] + col[tl],
+// per pair.  (Visiting pair (t + w) mod P instead needs a select per pair where
+// t + w carries into the next row, on the half-rate ALU: a Newton phase of 3
+// steps at L=232, q=21, 2^20 -- four energy passes, a count and three weighted
+// passes -- took 44.3 ms that way, 38.6 ms without.)  An exclusive or, and not
+// a rotation, because it maps every aligned group of 2^k steps to an aligned
+// group of sites: floats added as a balanced tree over the steps then have the
+// same sum in every lane.  B >= 8.
 
-// byte k of o = byte (k + r) mod B of w, for 0 <= r < B
+// byte k of o = byte (k ^ r) of w, for 0 <= r < B
 template <int B>
-__device__ __forceinline__ void rotate_block(const uint32_t (&w)[B / 4], uint32_t r, uint32_t (&o)[B / 4]) {
+__device__ __forceinline__ void permute_block(const uint32_t (&w)[B / 4], uint32_t r, uint32_t (&o)[B / 4]) {
     constexpr int W = B / 4;
-    const uint32_t rw = r >> 2, rb = 8 * (r & 3);
-    uint32_t t[W];
+    const uint32_t order = 0x3210u ^ (0x1111u * (r & 3));
 #pragma unroll
-    for (int k = 0; k < W; ++k) {
-        uint32_t v = w[0];
+    for (int k = 0; k < W; ++k) o[k] = __byte_perm(w[k], 0, order);
 #pragma unroll
-        for (int j = 1; j < W; ++j) v = ((k + rw) % W == (uint32_t)j) ? w[j] : v;
-        t[k] = v;
+    for (int s = 1; s < W; s <<= 1) {
+        uint32_t t[W];
+#pragma unroll
+        for (int k = 0; k < W; ++k) t[k] = (r & (4 * s)) ? o[k ^ s] : o[k];
+#pragma unroll
+        for (int k = 0; k < W; ++k) o[k] = t[k];
     }
-#pragma unroll
-    for (int k = 0; k < W; ++k) o[k] = __funnelshift_r(t[k], t[(k + 1) % W], rb);
 }
 
 // ---------------------------------------------------------------- consensus

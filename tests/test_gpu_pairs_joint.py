@@ -61,6 +61,29 @@ def test_pair_kernels_at_tile_edges(cuda, L, q, N):
         np.testing.assert_array_equal(host(out2), host(out))
 
 
+@pytest.mark.parametrize("q", QS)
+@pytest.mark.parametrize("L", [33, 65])
+def test_equal_sequences_have_equal_energies(cuda, L, q):
+    """A sequence's energy depends on its residues alone, not on the lane or the
+    chunk that sums it: copies tie, and share their average rank."""
+    rng = np.random.default_rng(100 * q + L)
+    J, kinds, N = random_model(L, q, q + L), 5, 4101
+    which = rng.integers(0, kinds, size=N)
+    which[:160] = np.repeat(np.arange(kinds), 32)  # each in every lane
+    mem = oracle.pack_seqs(rng.integers(0, q, size=(kinds, L)).astype("<u1")[which])
+    dm, dJ = dev(mem), dev(J)
+    E, r = empty((N,), np.float32), empty((N,), np.float32)
+    ws = empty((N + 1,), np.int64)
+    _lib.call("mi3_energies", dJ.data_ptr(), dm.data_ptr(), N, N, E.data_ptr(), L, q, ws.data_ptr(), ws.numel() * 8,
+              stream())
+    e = host(E)
+    for k in range(kinds):
+        assert np.unique(e[which == k]).size == 1
+    ws = empty((int(_lib.query("mi3_rank_workspace", N)) // 8 + 2,), np.int64)
+    _lib.call("mi3_rank_average", E.data_ptr(), N, r.data_ptr(), ws.data_ptr(), ws.numel() * 8, stream())
+    np.testing.assert_array_equal(host(r), oracle.rank_average(e).astype("<f4"))
+
+
 @pytest.mark.parametrize("q", [3, 5, 8, 21])
 def test_residues_past_the_alphabet_count_as_the_last(cuda, q):
     """Invalid residues (>= q) are clamped, as the pair kernels always did."""
