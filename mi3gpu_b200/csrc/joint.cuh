@@ -267,7 +267,7 @@ template <typename C>
 static JointGeom joint_geom(uint32_t L, uint32_t nseq) {
     JointGeom g;
     joint_slices(L, C::B, C::GI, C::GJ, &g);
-    g.chunk = pick_chunk(g.nslices, nseq, 148 * (1024 / C::T), 0xffffff00u, C::OVERHEAD, 1);
+    g.chunk = pick_chunk(g.nslices, nseq, 148 * (1024 / C::T), C::OVERHEAD);
     g.nchunks = (nseq - 1) / g.chunk + 1;
     return g;
 }

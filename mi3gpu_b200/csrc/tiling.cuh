@@ -48,28 +48,25 @@ inline uint32_t pick_block(uint32_t q, size_t budget, uint32_t max_b = 32) {
     return 0;
 }
 
-// Chunk length by a wave model: nslices * nchunks CTAs run 2 per SM, so the
-// time goes as ceil(CTAs / 296) * (chunk + overhead), where staging and
-// flushing a slice's table costs about as much as PAIR_CTA_OVERHEAD sequences.
-// (Targeting a fixed number of CTAs instead left last waves nearly empty:
-// 2080 CTAs = 7.03 waves at L=512, q=21, 2^18 sequences.)
-// For each number of waves only the largest nchunks that fits it is tried,
-// from min_waves on (PAIR_MIN_WAVES where slices differ in cost, which several
-// CTAs per slot even out).
-constexpr uint32_t PAIR_RESIDENT = 148 * 2, PAIR_CTA_OVERHEAD = 2048, PAIR_MIN_CHUNK = 1024, PAIR_MIN_WAVES = 3;
+// CTAs of 512 threads on the device, and the shortest chunk of sequences for one.
+constexpr uint32_t PAIR_RESIDENT = 148 * 2, PAIR_MIN_CHUNK = 1024;
 
-inline uint32_t pick_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident, uint32_t max_chunk,
-                           uint32_t overhead, uint32_t min_waves) {
-    const uint32_t min_chunk = std::min(PAIR_MIN_CHUNK, max_chunk);
-    const uint32_t least = (nseq - 1) / max_chunk + 1;  // chunks that max_chunk asks for
-    const uint32_t most = std::max(least, (nseq - 1) / min_chunk + 1);
-    auto chunk_of = [&](uint32_t nc) { return std::min(max_chunk, ((nseq - 1) / nc + 1 + 255) & ~255u); };
-    uint32_t pick = chunk_of(least);
+// Chunk length of the joint kernels (joint.cuh) by a wave model: nslices *
+// nchunks CTAs run `resident` at a time, so the time goes as ceil(CTAs /
+// resident) * (chunk + overhead), where staging and flushing a slice's table
+// costs about as much as `overhead` sequences.  (Targeting a fixed number of CTAs
+// instead left last waves nearly empty: 2080 CTAs = 7.03 waves at L=512, q=21,
+// 2^18 sequences.)  For each number of waves only the largest nchunks that fits
+// it is tried.
+inline uint32_t pick_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident, uint32_t overhead) {
+    const uint32_t most = (nseq - 1) / PAIR_MIN_CHUNK + 1;
+    auto chunk_of = [&](uint32_t nc) { return std::min(0xffffff00u, ((nseq - 1) / nc + 1 + 255) & ~255u); };
+    uint32_t pick = chunk_of(1);
     uint64_t best = ~0ull;
-    const uint32_t w0 = (uint32_t)(((uint64_t)nslices * least + resident - 1) / resident);
-    for (uint32_t w = std::max(w0, min_waves); w < w0 + 24; ++w) {
+    const uint32_t w0 = (nslices + resident - 1) / resident;
+    for (uint32_t w = w0; w < w0 + 24; ++w) {
         const uint64_t fit = (uint64_t)w * resident / nslices;
-        const uint32_t chunk = chunk_of((uint32_t)std::min<uint64_t>(std::max<uint64_t>(fit, least), most));
+        const uint32_t chunk = chunk_of((uint32_t)std::min<uint64_t>(std::max<uint64_t>(fit, 1), most));
         const uint64_t cost = w * ((uint64_t)chunk + overhead);
         if (cost < best) {
             best = cost;
@@ -80,12 +77,33 @@ inline uint32_t pick_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident, u
     return pick;
 }
 
+// Chunk length of the pair-major kernels, whose slices differ in cost: the work
+// spread over the device, plus half a CTA's for the tail.  A CTA costs about 640
+// sequences beside its chunk, and takes 1024 at a time.  Against the wave model
+// above, energies: L=12, q=4, 2^20 117 -> 90 us, L=64, q=24, 4096 27 -> 22 us;
+// against 8 CTAs per SM in chunks of 2048 or more: L=20, q=4, 10^5 51 -> 39 us,
+// counts L=187, q=24, 4096 63 -> 45 us.
+inline uint32_t pick_chunk_uneven(uint32_t nslices, uint32_t nseq, uint32_t resident) {
+    uint32_t pick = PAIR_MIN_CHUNK;
+    double best = 1e300;
+    for (uint64_t c = 1024; c < (1ull << 32); c += std::max<uint64_t>(1024, (c / 4) & ~1023ull)) {
+        const uint64_t chunks = (nseq - 1) / c + 1;
+        const double cost = ((double)nslices * chunks / resident + 0.5) * ((double)std::min<uint64_t>(c, nseq) + 640);
+        if (cost < best) {
+            best = cost;
+            pick = (uint32_t)c;
+        }
+        if (c >= nseq) break;
+    }
+    return pick;
+}
+
 inline SliceGeom make_geom(uint32_t L, uint32_t B, uint32_t nseq) {
     SliceGeom g;
     g.B = B;
     g.nb = (L + B - 1) / B;
     g.nslices = g.nb * (g.nb + 1) / 2;
-    g.chunk = pick_chunk(g.nslices, nseq, PAIR_RESIDENT, 0xffffff00u, PAIR_CTA_OVERHEAD, PAIR_MIN_WAVES);
+    g.chunk = pick_chunk_uneven(g.nslices, nseq, PAIR_RESIDENT);
     g.nchunks = (nseq - 1) / g.chunk + 1;
     return g;
 }
