@@ -178,12 +178,10 @@ __global__ void __launch_bounds__(T, 1024 / T) k_energies_joint(const float *__r
     } else {
         float *raw = js + joint_table(q, B, GI, GJ);
         const uint32_t S = joint_stage_pair(q, GJ), R = joint_stage_row(q, B, GJ);
-#pragma unroll 4
-        for (uint32_t t = warp; t < GI * B * GJ * B; t += nwarps) {
-            const uint32_t r = t / (GJ * B), cc = t % (GJ * B), i = i0 + r, j = j0 + cc;
-            const bool ok = i < j && j < L;
-            for (uint32_t e = lane; e < qq; e += 32) raw[r * R + cc * S + e] = ok ? __ldg(&J[pair_index(i, j, L) * qq + e]) : 0.0f;
-        }
+        joint_pairs<B, GI, GJ, T, QC>([&](uint32_t r, uint32_t cc, uint32_t e) {
+            const uint32_t i = i0 + r, j = j0 + cc;
+            raw[r * R + cc * S + e] = i < j && j < L ? __ldg(&J[pair_index(i, j, L) * qq + e]) : 0.0f;
+        });
         __syncthreads();
         // each cell: the float sum of its (at most four) site pairs' couplings
         for (uint32_t c = warp; c < QI * QJ; c += nwarps) {

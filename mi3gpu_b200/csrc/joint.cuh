@@ -72,19 +72,19 @@ __host__ __device__ constexpr uint32_t joint_states(uint32_t q, uint32_t G) { re
 // built or taken apart (G > 1 only).  The staging strides -- S per pair
 // (= 2 mod 16 for GJ = 2, 4 mod 32 for GJ = 1) and an odd row -- keep the 32
 // pairs of a warp on different banks (two lanes a bank at most).
-__host__ __device__ inline uint32_t joint_table(uint32_t q, uint32_t B, uint32_t GI, uint32_t GJ) {
+__host__ __device__ constexpr uint32_t joint_table(uint32_t q, uint32_t B, uint32_t GI, uint32_t GJ) {
     return joint_states(q, GI) * joint_states(q, GJ) * B * B;
 }
-__host__ __device__ inline uint32_t joint_stage_pair(uint32_t q, uint32_t GJ) {
+__host__ __device__ constexpr uint32_t joint_stage_pair(uint32_t q, uint32_t GJ) {
     return GJ == 2 ? ((q * q + 13) / 16) * 16 + 2 : ((q * q + 27) / 32) * 32 + 4;
 }
-__host__ __device__ inline uint32_t joint_stage_row(uint32_t q, uint32_t B, uint32_t GJ) {
+__host__ __device__ constexpr uint32_t joint_stage_row(uint32_t q, uint32_t B, uint32_t GJ) {
     return B * GJ * joint_stage_pair(q, GJ) + 1;
 }
-__host__ __device__ inline uint32_t joint_stage(uint32_t q, uint32_t B, uint32_t GI, uint32_t GJ) {
+__host__ __device__ constexpr uint32_t joint_stage(uint32_t q, uint32_t B, uint32_t GI, uint32_t GJ) {
     return GI * GJ == 1 ? 0 : GI * B * joint_stage_row(q, B, GJ);
 }
-inline size_t joint_smem(uint32_t q, uint32_t B, uint32_t GI, uint32_t GJ) {
+__host__ __device__ constexpr size_t joint_smem(uint32_t q, uint32_t B, uint32_t GI, uint32_t GJ) {
     return ((size_t)joint_table(q, B, GI, GJ) + joint_stage(q, B, GI, GJ)) * 4;
 }
 
@@ -235,15 +235,36 @@ __device__ __forceinline__ void slice_transpose(V *table, uint32_t qq, F &&fn) {
     }
 }
 
+// fn(row, column, entry) for all entries of a slice's GI*B x GJ*B site pairs, in
+// the order of the packed arrays: a warp takes a site pair at a time, or, where
+// that would leave half its lanes idle (q <= 4), the CTA takes consecutive entries
+// (L=64, 4096 sequences, energies: q=2 36 -> 23 us, q=3 37 -> 25; counts at q=5 and
+// 7 took 6 to 15% longer that way).
+template <int B, int GI, int GJ, int T, int QC, typename F>
+__device__ __forceinline__ void joint_pairs(F &&fn) {
+    constexpr uint32_t qq = QC * QC, row = GJ * B * qq;
+    if constexpr (qq <= 16) {
+#pragma unroll 4
+        for (uint32_t t = threadIdx.x; t < GI * B * row; t += T) fn(t / row, t % row / qq, t % qq);
+    } else {
+#pragma unroll 4
+        for (uint32_t t = threadIdx.x >> 5; t < GI * B * GJ * B; t += T / 32)
+            for (uint32_t e = threadIdx.x & 31; e < qq; e += 32) fn(t / (GJ * B), t % (GJ * B), e);
+    }
+}
+
 // Tile configuration of an alphabet: B joint sites per block, GI x GJ sites
-// per joint pair, T threads (1024 resident threads per SM at 64 registers,
-// so T = 1024 where one table fills the SM), and the alphabet QC where joint
+// per joint pair, T threads (1024 resident threads per SM at 64 registers, so T =
+// 1024 where table and staging of two CTAs exceed the SM: q=3, 2^16 sequences,
+// L=187, energies 121 us with 512, 78 with 1024; q=7, L=128, 85 and 72), and the alphabet QC where joint
 // states are packed and split, so that those divisions and sums unroll (0: any).
 // OVERHEAD: what building or splitting a CTA's table costs, in sequences.
 template <int B_, int GI_, int GJ_, int T_, int QC_>
 struct JointCfg {
     static constexpr int B = B_, GI = GI_, GJ = GJ_, T = T_, QC = QC_;
     static constexpr uint32_t OVERHEAD = GI * GJ == 1 ? 2048 : 4096;
+    // 1024 resident threads per SM, whose 228 KB hold their tables (and 1 KB a CTA)
+    static_assert(GI * GJ == 1 || (1024 / T) * (joint_smem(QC, B, GI, GJ) + 1024) <= 228 * 1024, "threads per CTA");
 };
 
 // Calls fn(JointCfg) for the alphabet; returns false when it has none.
@@ -251,11 +272,11 @@ template <typename F>
 static bool joint_dispatch(uint32_t q, F &&fn) {
     if (q == 1 || q == 9 || q == 10) fn(JointCfg<16, 1, 1, 512, 0>());
     else if (q == 2) fn(JointCfg<16, 2, 2, 512, 2>());
-    else if (q == 3) fn(JointCfg<16, 2, 2, 512, 3>());
+    else if (q == 3) fn(JointCfg<16, 2, 2, 1024, 3>());
     else if (q == 4) fn(JointCfg<8, 2, 2, 512, 4>());
     else if (q == 5) fn(JointCfg<8, 2, 2, 1024, 5>());
     else if (q == 6) fn(JointCfg<8, 2, 1, 512, 6>());
-    else if (q == 7) fn(JointCfg<8, 2, 1, 512, 7>());
+    else if (q == 7) fn(JointCfg<8, 2, 1, 1024, 7>());
     else if (q == 8) fn(JointCfg<8, 2, 1, 1024, 8>());
     else if (q >= 11 && q <= 21) fn(JointCfg<8, 1, 1, 512, 0>());
     else return false;

@@ -200,11 +200,10 @@ __global__ void __launch_bounds__(T, 1024 / T) k_pairhist_joint(const uint32_t *
             }
         }
         __syncthreads();
-        for (uint32_t t = warp; t < GI * B * GJ * B; t += nwarps) {
-            const uint32_t r = t / (GJ * B), cc = t % (GJ * B), i = i0 + r, j = j0 + cc;
-            if (!(i < j && j < L)) continue;
-            for (uint32_t e = lane; e < qq; e += 32) flush(pair_index(i, j, L) * qq + e, raw[r * R + cc * S + e]);
-        }
+        joint_pairs<B, GI, GJ, T, QC>([&](uint32_t r, uint32_t cc, uint32_t e) {
+            const uint32_t i = i0 + r, j = j0 + cc;
+            if (i < j && j < L) flush(pair_index(i, j, L) * qq + e, raw[r * R + cc * S + e]);
+        });
     }
 }
 
