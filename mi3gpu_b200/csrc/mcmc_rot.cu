@@ -73,6 +73,7 @@
 // 50688 1.0e10, 1.8e10; L=232 q=21 2^20 8.7e9, 1.16e10; L=512 q=21 2^18 3.2e9,
 // 3.7e9 (the fill: 0.9 MB of couplings per step for 448 walkers).
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -781,23 +782,36 @@ static uint32_t rot_slots(const RotShape &r, const RotPick &k, uint32_t warps) {
     return 0;
 }
 
-// SM cycles per step of a CTA of w warps, times the waves of CTAs: the
-// largest of its instructions (at 3.2 a cycle), its gathers plus the fill through
-// shared memory (64 bytes a cycle), one warp's own chain (4.2 cycles an
-// instruction; 200 more per exchange between a walker's lanes), and the fill's
-// way from L2 (48 bytes a cycle and SM when all SMs pull).  Against a sweep of
-// all (lanes, warps) over ten shapes from L=20 to 512 the plan it picks was
-// within 3% of the fastest.
+// SM cycles per step of all walkers with CTAs of w warps: as many CTAs share an
+// SM as its memory and registers hold (8% more where they do, since small CTAs
+// end raggedly), and a wave of them takes about the largest (the 3-norm) of their
+// instructions (at 3 a cycle), their gathers plus half the fill through shared
+// memory, and one warp's own chain (the waits of a chunk, and 20 to 25 cycles a
+// term, 43 with 5-bit fields; more per chunk where lanes share a walker).  Fitted
+// to 6000 timed (lanes, warps) of 140 shapes from L=48 to 570, of which the plan it
+// picks is 1.3% slower than the fastest in the mean; the largest of the three with
+// a chain half as long and one CTA per SM, taken before, was 6% slower in the mean
+// and 45% at worst (L=256, q=21, 2^17 walkers: 1.57 ms per 64 steps, now 1.08;
+// L=232, q=21, 65536: 0.71, now 0.54).
 static double rot_cost(const RotShape &r, const RotPick &k, uint32_t w, uint32_t nseqs) {
+    const bool diff = r.mode == ROT_DIFF2, late = k.nw > 40 && k.nw < 64;
     const double steps = k.S == 1 ? 32 * (r.nc - 1) + r.tail : 32.0 / k.S * r.nc;
-    const double gathers = r.mode == ROT_DIFF2 ? 1 : 2, share = k.S == 1 ? 0 : k.S == 2 ? 1 : 2;
-    const double instr =
-        steps * (r.mode == ROT_DIFF2 ? 2.5 : k.bits == 8 ? 5.0 : 6.7) + 35.0 * r.nc + 240.0 + 20.0 * share;
-    const double fill = 2.0 * r.nc * r.cells;
-    const uint32_t per_cta = w * 32 / k.S, waves = ((nseqs + per_cta - 1) / per_cta + 147) / 148;
-    double t = std::max(w * instr / 3.2, w * gathers * steps + fill);
-    t = std::max(t, std::max(4.2 * instr + 250.0 + 200.0 * share + 12.0 * w, fill * 64.0 / 48.0));
-    return waves * t;
+    const double share = k.S == 1 ? 0 : k.S == 2 ? 1 : 2;
+    const double instr = diff ? steps * 2.5 + 120.0 * r.nc + 228.0
+                              : steps * (k.bits == 8 ? 5.0 : 6.7) + 95.0 * r.nc + 200.0;
+    const double chain =
+        steps * (diff ? 20.0 : k.bits == 8 ? 25.0 : 43.0) + r.nc * ((diff ? 600.0 : 780.0) + 110.0 * share) + 705.0;
+    auto wave = [&](uint32_t ctas) {
+        const double issue = ctas * w * instr / (diff ? 2.9 : 3.1);
+        const double smem = ctas * (w * (diff ? 1 : 2) * steps + (double)r.nc * r.cells);
+        return std::cbrt(issue * issue * issue + smem * smem * smem + chain * chain * chain) * (late ? 1.15 : 1.0);
+    };
+    const uint32_t regs = 65536 / k.maxt / 8 * 8, per_cta = w * 32 / k.S, ctas = (nseqs + per_cta - 1) / per_cta;
+    const uint32_t fit = std::min((uint32_t)(228 * 1024 / (rot_smem(r, k, w, rot_slots(r, k, w)) + 1024)),
+                                  std::min(65536 / (regs * 32 * w), 2048 / (32 * w)));
+    const uint32_t per_sm = std::max(1u, fit), waves = ctas / (148 * per_sm), rest = ctas - waves * 148 * per_sm;
+    const double t = waves * wave(per_sm) + (rest ? wave((rest + 147) / 148) : 0.0);
+    return per_sm > 1 && ctas > 148 ? 1.08 * t : t;
 }
 
 // Lanes per walker and warps per CTA (fixed ones, or 0: the cheapest).
