@@ -788,12 +788,13 @@ static uint32_t rot_slots(const RotShape &r, const RotPick &k, uint32_t warps) {
 // instructions (at 3 a cycle), their gathers plus half the fill through shared
 // memory, and one warp's own chain (the waits of a chunk, and 20 to 25 cycles a
 // term, 43 with 5-bit fields; more per chunk where lanes share a walker).  Fitted
-// to 6000 timed (lanes, warps) of 140 shapes from L=48 to 570, of which the plan it
-// picks is 1.3% slower than the fastest in the mean; the largest of the three with
-// a chain half as long and one CTA per SM, taken before, was 6% slower in the mean
-// and 45% at worst (L=256, q=21, 2^17 walkers: 1.57 ms per 64 steps, now 1.08;
+// to 6000 timed (lanes, warps) of 140 shapes from L=48 to 570, of which the plan
+// rot_plan picks is 1.8% slower alone than the fastest in the mean; the largest of
+// the three with a chain half as long and one CTA per SM, taken before, was 6%
+// slower in the mean and 45% at worst (L=256, q=21, 2^17 walkers: 1.57 ms per 64 steps, now 1.08;
 // L=232, q=21, 65536: 0.71, now 0.54).
-static double rot_cost(const RotShape &r, const RotPick &k, uint32_t w, uint32_t nseqs) {
+// work: the instructions' share of it, were all SMs full.
+static double rot_cost(const RotShape &r, const RotPick &k, uint32_t w, uint32_t nseqs, double &work) {
     const bool diff = r.mode == ROT_DIFF2, late = k.nw > 40 && k.nw < 64;
     const double steps = k.S == 1 ? 32 * (r.nc - 1) + r.tail : 32.0 / k.S * r.nc;
     const double share = k.S == 1 ? 0 : k.S == 2 ? 1 : 2;
@@ -811,10 +812,15 @@ static double rot_cost(const RotShape &r, const RotPick &k, uint32_t w, uint32_t
                                   std::min(65536 / (regs * 32 * w), 2048 / (32 * w)));
     const uint32_t per_sm = std::max(1u, fit), waves = ctas / (148 * per_sm), rest = ctas - waves * 148 * per_sm;
     const double t = waves * wave(per_sm) + (rest ? wave((rest + 147) / 148) : 0.0);
+    work = (double)ctas * w * instr / (diff ? 2.9 : 3.1) / 148;
     return per_sm > 1 && ctas > 148 ? 1.08 * t : t;
 }
 
-// Lanes per walker and warps per CTA (fixed ones, or 0: the cheapest).
+// Lanes per walker and warps per CTA (fixed ones, or 0: the cheapest).  A plan is
+// also charged 0.4 of its work: one problem that does not fill the device may have
+// others beside it, and more lanes per walker are more instructions (three problems
+// of L=48, q=4, 2^14 walkers in turn, 768 proposals: 339 us each at two lanes, 278
+// at one, though two are 4% faster alone).
 static RotPick rot_plan(const RotShape &r, uint32_t nseqs, uint32_t walkers, uint32_t lanes, uint32_t &warps) {
     RotPick pick{nullptr, 0, 0, 0, 0};
     double best = 1e300;
@@ -825,7 +831,8 @@ static RotPick rot_plan(const RotShape &r, uint32_t nseqs, uint32_t walkers, uin
         for (uint32_t w = 1; w <= k.maxt / 32; ++w) {
             if (walkers && w * 32 != walkers * S) continue;
             if (!rot_slots(r, k, w)) continue;
-            const double c = rot_cost(r, k, w, nseqs);
+            double work;
+            const double t = rot_cost(r, k, w, nseqs, work), c = t + 0.4 * work;
             if (c < 0.999 * best) {
                 best = c;
                 pick = k;
