@@ -168,6 +168,11 @@ int mi3_metropolis_rot(const float *Jrot, uint32_t *rngstates, uint32_t position
                        uint32_t *seqmem, uint32_t nseqs, uint32_t L, uint32_t q, uint32_t walkers_per_cta,
                        uint32_t lanes_per_walker, int32_t *status, void *stream);
 
+/* 1 where mi3_metropolis_rot with its own choice of plan is expected to take no
+ * longer than mi3_metropolis with its own for these sizes, else 0 (models of both,
+ * host only; the time of unpacking is left out). */
+uint32_t mi3_metropolis_rot_pays(uint32_t L, uint32_t q, uint32_t nseqs);
+
 /* gen_indep (mcmc.cl:170-244) as launched by MCMCGPU.gen_indep
  * (mcmcGPU.py:380-390); cprob is (L, q-1) cumulative probabilities
  * (MCMCGPU.prepare_indep, mcmcGPU.py:375-378). */

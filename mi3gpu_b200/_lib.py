@@ -42,6 +42,7 @@ SIGNATURES = {
     "mi3_unpack_j_rot": (c.c_int, [_vp, _vp, _u32, _u32, _vp]),
     "mi3_metropolis_rot": (c.c_int, [_vp, _vp, _u32, _vp, _u32, _vp, _f32, _vp, _u32, _u32, _u32, _u32, _u32, _vp,
                                      _vp]),
+    "mi3_metropolis_rot_pays": (_u32, [_u32, _u32, _u32]),
     "mi3_gen_indep": (c.c_int, [_vp, _u32, _u32, _vp, _vp, _u32, _u32, _vp]),
     "mi3_energies_workspace": (c.c_size_t, [_u32]),
     "mi3_energies": (c.c_int, [_vp, _vp, _u32, _u32, _vp, _u32, _u32, _vp, c.c_size_t, _vp]),

@@ -83,6 +83,8 @@ constexpr uint32_t ROT_HEAD = 256;  // mbarriers, copy counts, abort flag
 constexpr uint32_t ROT_MAX_SLOTS = 6;
 constexpr uint64_t ROT_JOINT_MAX = 96ull << 20;  // bytes of a joint table
 
+double metro_cycles(uint32_t L, uint32_t q, uint32_t nseqs);  // mcmc.cu
+
 enum RotMode { ROT_PAIR1 = 0, ROT_PAIR2 = 1, ROT_DIFF2 = 2 };
 
 struct RotShape {
@@ -850,6 +852,23 @@ using namespace mi3;
 extern "C" uint64_t mi3_jrot_floats(uint32_t L, uint32_t q) {
     RotShape r;
     return rot_shape(L, q, r) ? r.words : 0;
+}
+
+// Both models' errors are about 5%; where one lane can hold a walker's row, rot_cost
+// is the higher one by up to 20%, hence the tenth.  Beyond, q <= 4 never pays: the
+// row kernel's gathers mostly broadcast there.  Of 150 shapes the rotated kernel was
+// slower than the row kernel at ten before this test, by up to 37% (L=503, q=4,
+// 23552 walkers).
+extern "C" uint32_t mi3_metropolis_rot_pays(uint32_t L, uint32_t q, uint32_t nseqs) {
+    RotShape r;
+    if (!rot_shape(L, q, r) || nseqs == 0 || nseqs % 32) return 0;
+    uint32_t warps = 0;
+    const RotPick k = rot_plan(r, nseqs, 0, 0, warps);
+    if (!k.kernel) return 0;
+    const bool one_lane = rot_kernel(r, 1).kernel != nullptr;
+    if (!one_lane && q <= 4) return 0;
+    double work;
+    return rot_cost(r, k, warps, nseqs, work) <= (one_lane ? 1.1 : 1.0) * metro_cycles(L, q, nseqs);
 }
 
 extern "C" int mi3_unpack_j_rot(const float *J, float *Jrot, uint32_t L, uint32_t q, void *stream) {

@@ -15,6 +15,7 @@ gives the same order.  `wait_for` arguments are accepted for signature
 compatibility; commands are always ordered after the previous command.
 """
 import collections
+import functools
 import time
 from pathlib import Path
 
@@ -25,6 +26,11 @@ import torch
 from . import _lib, seqload
 
 rng_buf_mul = 1024  # position-list blocks of 1024*nsteps (mcmcGPU.py:30)
+
+
+@functools.lru_cache(maxsize=256)
+def _rot_pays(L, q, nseqs):
+    return bool(_lib.query('mi3_metropolis_rot_pays', L, q, nseqs))
 
 
 def _full_shape(buftype, bufshape):
@@ -498,8 +504,16 @@ class MCMCGPU:
         own (in brackets one problem alone): L=100 q=4 8192 walkers 1.13
         (1.18), 49152 1.21 (1.74); q=8 16384 0.61 (1.03), 49152 1.04 (1.51);
         q=21 8192 0.81 (1.04), 49152 1.16 (1.62); L=37 q=8 49152 0.80 (1.12),
-        L=37 q=4 8192 0.93 (1.02), L=48 q=4 16384 1.14 (1.04)."""
-        return self.L >= (48 if self.q <= 5 else 64) and (self.q <= 5 or self.nseq['main'] >= 49152)
+        L=37 q=4 8192 0.93 (1.02), L=48 q=4 16384 1.14 (1.04).  Within those
+        lines, where both kernels' models say that it pays against the row
+        kernel (mi3_metropolis_rot_pays: not on long rows at q <= 4, nor where
+        a last wave of CTAs is nearly empty).  Against the skewed-lane kernel,
+        where that would run instead, it is not weighed: 51 shapes took 0.86
+        to 2.2 times as long there, eight of them less than 1."""
+        L, q, N = self.L, self.q, self.nseq['main']
+        if not (L >= (48 if q <= 5 else 64) and (q <= 5 or N >= 49152)):
+            return False
+        return self.sampler_plan()[0] == 'skew' or _rot_pays(L, q, N)
 
     def sampler_kernel(self):
         """The sampler runMCMC runs: 'rot' (mi3_metropolis_rot) or 'plan' (the

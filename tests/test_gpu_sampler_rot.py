@@ -159,7 +159,7 @@ def test_rot_bad_site_reported_and_shapes_refused(cuda):
                       buf.data_ptr(), N, L, q, wpc, lanes, status.data_ptr(), stream())
 
 
-@pytest.mark.parametrize("L,q,kind", [(47, 4, "plan"), (48, 4, "rot"), (64, 6, "plan")])
+@pytest.mark.parametrize("L,q,kind", [(47, 4, "plan"), (48, 4, "rot"), (64, 6, "plan"), (400, 4, "plan")])
 def test_untuned_choice_keeps_the_trajectories(cuda, L, q, kind):
     """Both sides of rot_default: the same walkers and generators as with the
     other kernel, bit for bit."""

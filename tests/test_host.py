@@ -630,6 +630,24 @@ def test_untuned_sampler_plan_dispatch():
     assert plan(99, 4, 1 << 18, tuned=['skew', 768]) == ('skew', 768)
 
 
+@pytest.mark.parametrize("L,q,N,kind", [
+    (48, 4, 512, 'rot'), (47, 4, 512, 'plan'), (93, 4, 1 << 18, 'rot'), (187, 8, 50688, 'rot'),
+    (187, 8, 49120, 'plan'),  # q > 5 and fewer than 49152 walkers
+    (380, 4, 32768, 'rot'), (400, 4, 32768, 'plan'), (512, 4, 131072, 'plan'),  # no joint table: long rows
+    (280, 8, 65536, 'rot'), (380, 9, 148480, 'plan'),  # a last wave nearly empty
+    (232, 21, 1 << 20, 'rot'), (576, 21, 1 << 18, 'rot'), (577, 21, 1 << 18, 'plan')])
+def test_untuned_sampler_kernel(L, q, N, kind):
+    """MCMCGPU.sampler_kernel without tuning, on both sides of its lines; an
+    installed plan or sampler_rot overrides it."""
+    g = MCMCGPU.__new__(MCMCGPU)
+    g.L, g.q, g.nseq = L, q, {'main': N}
+    assert g.sampler_kernel() == kind
+    g.metro_plan = (512, 24, 3)
+    assert g.sampler_kernel() == 'plan'
+    g.sampler_rot = True
+    assert g.sampler_kernel() == ('rot' if L <= 576 else 'plan')
+
+
 @pytest.mark.parametrize("L,q,sigma", [(48, 4, 0.5), (60, 21, 0.5), (99, 4, 0.8)])
 def test_synthetic_ground_truth_matches_its_definition(L, q, sigma):
     """The benchmark workloads' ground truth (fields N(0,1), couplings
