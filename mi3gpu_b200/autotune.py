@@ -100,17 +100,19 @@ class Autotuner:
 
     def sampler_rot(self, gpu, probe_steps=None, reps=2):
         """Whether the rotated sampler beats the best plan of sampler_plan for
-        gpu's shape, timed the same way."""
+        gpu's shape.  Both are timed here: the times in the table may be those
+        of another number of proposals."""
         if not gpu.rot_supported():
             return False
-        plan, ms = self.sampler_plan(gpu, probe_steps, reps)
+        plan, _ = self.sampler_plan(gpu, probe_steps, reps)
         key = self._key("metropolis_rot", gpu)
-        if key not in self.table:
+        if "probe_steps" not in self.table.get(key, {}):
             gpu.require('MCMC')
             gpu.unpackJ(kind='rot')
-            times, _ = self._time_sampler(gpu, [('rot',)], probe_steps, reps)
-            best = ms.get(_plan_key(plan))
-            self.table[key] = {"ms": times[('rot',)], "use": best is None or times[('rot',)] <= best}
+            gpu.unpackJ(kind='tiles' if plan[0] == 'skew' else 'rows')
+            times, steps = self._time_sampler(gpu, [('rot',), plan], probe_steps, reps)
+            self.table[key] = {"ms": times[('rot',)], "plan_ms": times[plan], "probe_steps": steps,
+                               "use": times[('rot',)] <= times[plan]}
             self._save()
         return bool(self.table[key]["use"])
 

@@ -372,6 +372,28 @@ def test_autotuner_cache_roundtrip_and_concurrent_writers(tmp_path):
     assert os.path.exists(path)
 
 
+@pytest.mark.parametrize("rot_ms,plan_ms", [(3.0, 2.0), (2.0, 3.0)])
+def test_autotuner_weighs_samplers_at_the_same_number_of_proposals(monkeypatch, rot_ms, plan_ms):
+    """A cached plan may have been timed with fewer or more proposals: the
+    choice of the rotated sampler times both anew, and a verdict without its
+    number of proposals is not believed."""
+    from types import SimpleNamespace
+    from mi3gpu_b200 import autotune
+    monkeypatch.setattr(autotune.torch.cuda, "get_device_name", lambda d: "fake")
+    gpu = SimpleNamespace(L=100, q=21, nseq={'main': 512}, device=None, rot_supported=lambda: True,
+                          require=lambda c: None, unpackJ=lambda kind: None)
+    t = autotune.Autotuner()
+    t.table[t._key("metropolis", gpu)] = {"plan": ["skew", 512], "ms": {"skew,512": 2.5}, "probe_steps": 7}
+    t.table[t._key("metropolis_rot", gpu)] = {"ms": 2.4, "use": rot_ms > plan_ms}
+    times = {('rot',): rot_ms, ('skew', 512): plan_ms}
+    monkeypatch.setattr(t, "_time_sampler", lambda g, plans, steps, reps: ({p: times[p] for p in plans}, 200))
+    assert t.sampler_rot(gpu) == (rot_ms <= plan_ms)
+    assert t.table[t._key("metropolis_rot", gpu)]["probe_steps"] == 200
+    times[('rot',)] = 9.0
+    assert t.sampler_rot(gpu) == (rot_ms <= plan_ms)  # from the table
+
+
+
 def _ckpt_run(tmp_path, rounds, dev, reseed, resume_from=None, ckpt_name="ck.pkl"):
     from mi3gpu_b200 import checkpoint
     L, q, N = 6, 3, 512
