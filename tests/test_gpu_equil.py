@@ -37,7 +37,7 @@ def _inputs(n, seed):
     yield np.full(n, 7.0, "<f4")               # constant
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 2047, 2048, 4097, 100003, 1 << 20])
+@pytest.mark.parametrize("n", [1, 2, 3, 2047, 2048, 4097, 100003, 1 << 20, (1 << 23) - 1])
 def test_rank_average_bitexact(cuda, n):
     for x in _inputs(n, n):
         _, r = _ranks(x)

@@ -26,7 +26,9 @@ def _phase(L, q, N, reg, regarg, fused, onecall, mode="all"):
     lines = []
     n, _, _ = NewtonSteps.iterNewton(p, None, node, lines.append, fused=fused)
     node.wait()
-    out = [g.getBuf(b).read() for b in ("J", "dJ", "bi", "weightstats64", "minout")]
+    seqbuf = "main" if mode == "all" else "large"
+    out = [g.getBuf(b).read() for b in ("J", "dJ", "bi", "weightstats64", "minout", "E " + seqbuf,
+                                        "weights" if mode == "all" else "weights large")]
     return n, out, [x for x in lines if "Neff" in x]
 
 
