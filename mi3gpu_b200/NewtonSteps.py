@@ -145,7 +145,7 @@ def iterNewton(param, bimarg_model, gpus, log, fused=False):
     # kernels; fused or not gives the same values)
     step = None
     if param.beta is None and hasattr(gpus, 'newtonStepper'):
-        step = gpus.newtonStepper(gamma, pc, param.reg, tuple(param.regarg or ()), seqbuf)
+        step = gpus.newtonStepper(gamma, pc, param.reg, tuple(param.regarg) if param.reg is not None else (), seqbuf)
     for i in range(newtonSteps):
         if step is not None:
             wsum, wsum2, mindE = step(ref_dE)

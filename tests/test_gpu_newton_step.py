@@ -48,6 +48,13 @@ def test_one_call_step_on_the_large_buffer(cuda):
         np.testing.assert_array_equal(x, y)
 
 
+@pytest.mark.parametrize("reg,regarg", [("SCADJ", (0.05, 0.5)), ("l1z", (2e-4,))])
+def test_regularizer_arguments_may_be_an_array(cuda, reg, regarg):
+    a, b = (_phase(20, 4, 1024, reg, r, True, True) for r in (regarg, np.array(regarg)))
+    for x, y in zip(a[1], b[1]):
+        np.testing.assert_array_equal(x, y)
+
+
 def test_one_call_step_takes_only_what_it_does(cuda):
     g = MCMCGPU((0, 0), 12, 4, 512, 512, None, 1024, 3)
     g.initJstep()
