@@ -275,8 +275,11 @@ __global__ void __launch_bounds__(STAT_THREADS) k_pair_stats(const float *__rest
 // (same order), elements e = lane + 32 k.  Each warp takes every (8 * CTAs)-th
 // pair, then a shuffle tree per statistic and a fixed-order sum over the CTA's
 // warps: one set of partials per CTA (at most STAT_CTAS), so that the last
-// reduction reads 57 KB and not 6 MB (L=512).  Entries above the threshold are
-// queued and divided 32 at a time: nearly every group of 32 entries has one.
+// reduction reads 57 KB and not 6 MB (L=512).  Each lane marks its entries above
+// the threshold in a word and divides them after the pass, in as many rounds as
+// the fullest lane has: nearly every group of 32 entries has one.  (A queue in
+// shared memory cost a CTA per SM at q=32: L=200 without J 109 us, now 58; L=512,
+// q=21 with J 363 and 356.)
 constexpr uint32_t STAT_CTAS = 148 * 8;
 
 __global__ void __launch_bounds__(256) k_pair_stats_w(const float *__restrict__ tgt, const float *__restrict__ mdl,
@@ -284,10 +287,9 @@ __global__ void __launch_bounds__(256) k_pair_stats_w(const float *__restrict__ 
                                                       uint32_t np) {
     __shared__ double sums[8][4][32];
     __shared__ double red[8][NSTAT];
-    extern __shared__ float stage[];  // [8 warps][2][q q]: the pair's target and model; then [8][q q] u16 queues
+    extern __shared__ float stage[];  // [8 warps][2][q q]: the pair's target and model
     const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31, qq = q * q;
     float *T = stage + (size_t)w * 2 * qq, *M = T + qq;
-    uint16_t *top = reinterpret_cast<uint16_t *>(stage + (size_t)16 * qq) + w * qq;
     double *ma = sums[w][0], *mb = sums[w][1], *ta = sums[w][2], *tb = sums[w][3];
     const uint32_t da = 32 / q, db = 32 - da * q;
     double v[NSTAT] = {0, 0, 0, 0, 0, 0};
@@ -310,17 +312,14 @@ __global__ void __launch_bounds__(256) k_pair_stats_w(const float *__restrict__ 
             ma[l] = sm_r; mb[l] = sm_c; ta[l] = st_r; tb[l] = st_c;
         }
         __syncwarp();
-        uint32_t ntop = 0, a = l / q, b = l - a * q;
+        uint32_t top = 0, a = l / q, b = l - a * q;  // top, bit k: entry 32 k + l
         for (uint32_t e0 = 0; e0 < qq; e0 += 32) {
             const uint32_t e = e0 + l;
             const bool in = e < qq;
             const double t = in ? T[e] : 0.0f, m = in ? M[e] : 0.0f, d = t - m;
             v[0] += d * d;
             v[1] = fmax(v[1], fabs(d));
-            const bool big = in && T[e] > 0.01f;
-            const uint32_t mask = __ballot_sync(0xffffffffu, big);
-            if (big) top[ntop + __popc(mask & ((1u << l) - 1u))] = (uint16_t)e;
-            ntop += __popc(mask);
+            if (in && T[e] > 0.01f) top |= 1u << (e0 >> 5);
             if (J && in) {
                 const double jv = J[(size_t)p * qq + e];
                 v[4] += jv * (m - ma[a] * mb[b]);
@@ -333,9 +332,9 @@ __global__ void __launch_bounds__(256) k_pair_stats_w(const float *__restrict__ 
                 ++a;
             }
         }
-        __syncwarp();
-        for (uint32_t k = l; k < ntop; k += 32) {
-            const double t = T[top[k]], m = M[top[k]];
+        for (; top; top &= top - 1) {
+            const uint32_t e = 32 * (__ffs(top) - 1) + l;
+            const double t = T[e], m = M[e];
             v[2] += fabs(t - m) / t;
             v[3] += 1.0;
         }
@@ -451,7 +450,7 @@ extern "C" int mi3_bimarg_stats(const float *target, const float *model, const f
     double *part = reinterpret_cast<double *>(workspace);
     uint32_t nparts = (uint32_t)np;
     if (q <= 32) {
-        const size_t sm = (size_t)8 * q * q * (2 * sizeof(float) + sizeof(uint16_t));
+        const size_t sm = (size_t)8 * 2 * q * q * sizeof(float);
         if (sm > 36 * 1024) cudaFuncSetAttribute(k_pair_stats_w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         nparts = std::min<uint32_t>((uint32_t)((np + 7) / 8), STAT_CTAS);
         k_pair_stats_w<<<nparts, 256, sm, st>>>(target, model, J, part, q, (uint32_t)np);
