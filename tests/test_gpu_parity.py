@@ -250,6 +250,18 @@ def test_bicounts_to_bimarg(cuda):
     np.testing.assert_array_equal(host(out), oracle.bicounts_to_bimarg(c, 4096))
 
 
+@pytest.mark.parametrize("shift", [0, 1])
+def test_bicounts_to_bimarg_four_entries_a_thread(cuda, shift):
+    """Enough entries for four a thread, two of them left over; with pointers off
+    the 16-byte lines, one a thread."""
+    L, q = 61, 17
+    n = L * (L - 1) // 2 * q * q
+    c = np.random.default_rng(5).integers(0, 4096, size=n + shift).astype(np.uint32)
+    out, dc = empty((n + shift,), np.float32), dev(c)
+    _lib.call("mi3_bicounts_to_bimarg", dc.data_ptr() + 4 * shift, out.data_ptr() + 4 * shift, 4096, L, q, stream())
+    np.testing.assert_array_equal(host(out)[shift:], c[shift:].astype(np.float32) / np.float32(4096))
+
+
 def test_update_j_bitexact(cuda):
     L, q = 40, 21
     rng = np.random.default_rng(12)
