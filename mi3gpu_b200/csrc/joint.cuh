@@ -28,10 +28,10 @@
 //
 // Measured against the pair-major tiling with lanes over pairs in full slices
 // only (Newton phases on one B200, l1z or l2z included):
-//   L=93  q=4  2^18  8 steps   10.0 -> 2.23 ms (2.92 with the alphabet a
+//   L=93  q=4  2^18  8 steps   10.0 -> 2.15 ms (2.92 with the alphabet a
 //                              run-time value in the packing and splitting)
-//   L=151 q=8  66048 8 steps   5.55 -> 2.87 ms (3.58)
-//   L=232 q=21 2^20  3 steps   38.6 -> 35.4 ms (edge slices, packed adds, one
+//   L=151 q=8  66048 8 steps   5.55 -> 2.88 ms (3.58)
+//   L=232 q=21 2^20  3 steps   38.6 -> 35.5 ms (edge slices, packed adds, one
 //                              clamp test per word)
 #pragma once
 #include "tiling.cuh"

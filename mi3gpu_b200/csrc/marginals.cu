@@ -300,57 +300,47 @@ constexpr uint32_t WMARG_CHUNK = 65536;  // sequences per CTA (fixed-point headr
 // Chunks of a weighted pass.  The chunk length also sets the fixed-point
 // scale (fixed_shift), so a pass is cut into at least the chunks that about 8
 // CTAs per SM of the pair-major tiling would take, and no chunk is longer than
-// WMARG_CHUNK.  The joint kernels may take more chunks: each costs a plane of
-// bins, written and read once (counted as 4096 sequences), against whole waves
-// of CTAs.  The number never falls as nseq grows (the plane term's weight falls).
-struct WmargSplit {
-    uint32_t chunks;    // asked for
-    uint32_t nslices;   // of the kernel that runs
-    uint32_t resident;  // its CTAs on the device
-};
-
-static WmargSplit wmarg_split(uint32_t L, uint32_t q, uint32_t nseq) {
+// WMARG_CHUNK.  Each chunk costs a plane of bins, written and read once
+// (counted as 4096 sequences), against whole waves of CTAs.  The number never
+// falls as nseq grows (the plane term's weight falls), so a workspace for nseq
+// sequences also serves fewer.
+// (Chunks of 2048 where this takes 1024 to 2047 are faster with small tables or
+// few sites -- L=64, q=8, 2^17 sequences 92 us against 121, L=48, q=21, 65536 69
+// against 111 -- but hold a bit less of each weight: 7.5e-8 of the bimarginals
+// against 4.3e-8 at L=64, q=21, 2^14.)
+static uint32_t wmarg_split(uint32_t L, uint32_t q, uint32_t nseq) {
     const uint32_t B = pick_block(q, 116 * 1024, 16);
-    if (!B) return WmargSplit{1, 1, 1};
+    if (!B) return 1;
     const uint32_t nb = (L + B - 1) / B, pair_slices = nb * (nb + 1) / 2;
     const uint32_t least = (148 * 8 + pair_slices - 1) / pair_slices;
-    WmargSplit sp{least, pair_slices, PAIR_RESIDENT};
-    const bool joint = joint_dispatch(q, [&](auto cfg) {
+    uint32_t ns = pair_slices, resident = PAIR_RESIDENT;
+    joint_dispatch(q, [&](auto cfg) {
         using C = decltype(cfg);
         JointGeom g;
         joint_slices(L, C::B, C::GI, C::GJ, &g);
-        sp.nslices = g.nslices;
-        sp.resident = 148 * (1024 / C::T);
+        ns = g.nslices;
+        // (q = 3 and 7 once ran 512 threads a CTA: their chunks, and with them
+        // the scale, are still those)
+        resident = q == 3 || q == 7 ? PAIR_RESIDENT : 148 * (1024 / C::T);
     });
-    if (!joint) return sp;
-    const uint32_t w0 = (least * sp.nslices + sp.resident - 1) / sp.resident;
+    const uint32_t w0 = (least * ns + resident - 1) / resident;
+    uint32_t best_k = least;
     double best = 1e30;
     for (uint32_t w = w0; w < w0 + 24; ++w) {
-        const uint32_t k = std::max(least, (uint32_t)((uint64_t)w * sp.resident / sp.nslices));
+        const uint32_t k = std::max(least, (uint32_t)((uint64_t)w * resident / ns));
         const double cost = (double)w / k * (1.0 + k * 4096.0 / nseq);
         if (cost < best) {
             best = cost;
-            sp.chunks = k;
+            best_k = k;
         }
     }
-    return sp;
-}
-
-// The shortest chunk worth a table and a plane of its own: 1024 sequences while
-// chunks of 2048 would fill less than a quarter of the device, else those.  In
-// chunks of 2048 a pass took, against 1024, 1.05 to 1.2 times as long below that
-// line and 0.85 to 0.95 times between it and a full device; beyond, L=64, q=8,
-// 2^17 sequences went from 120 us in chunks of 1280 to 91.
-static uint32_t least_chunk(uint32_t nslices, uint32_t nseq, uint32_t resident) {
-    const uint64_t ctas = (uint64_t)nslices * ((nseq - 1) / (2 * PAIR_MIN_CHUNK) + 1);
-    return 4 * ctas >= resident ? 2 * PAIR_MIN_CHUNK : PAIR_MIN_CHUNK;
+    return best_k;
 }
 
 uint32_t wmarg_fixed_chunk(uint32_t L, uint32_t q, uint32_t nseq) {
     if (!nseq) return WMARG_CHUNK;
-    const WmargSplit sp = wmarg_split(L, q, nseq);
-    const uint32_t chunk = ((nseq - 1) / sp.chunks + 1 + 255) & ~255u;
-    return std::min(std::max(chunk, least_chunk(sp.nslices, nseq, sp.resident)), WMARG_CHUNK);
+    const uint32_t chunk = ((nseq - 1) / wmarg_split(L, q, nseq) + 1 + 255) & ~255u;
+    return std::min(std::max(chunk, PAIR_MIN_CHUNK), WMARG_CHUNK);
 }
 
 template <int B, bool WEIGHTED>
@@ -707,7 +697,7 @@ extern "C" int mi3_bicounts(const uint32_t *seqmem, uint32_t buflen, uint32_t ns
 
 extern "C" size_t mi3_weighted_marg_workspace(uint32_t L, uint32_t q, uint32_t nseq) {
     // at least the chunks of any call with up to nseq sequences
-    const uint32_t split = nseq ? std::min(wmarg_split(L, q, nseq).chunks, nseq / PAIR_MIN_CHUNK + 1) : 1;
+    const uint32_t split = nseq ? std::min(wmarg_split(L, q, nseq), nseq / PAIR_MIN_CHUNK + 1) : 1;
     const uint32_t nchunks = std::max(nseq / WMARG_CHUNK + 1, split);
     return 256 + usite_bytes(L, q) + (size_t)nchunks * npairs_of(L) * q * q * 4;
 }
