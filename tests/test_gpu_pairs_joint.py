@@ -32,8 +32,9 @@ def test_pair_kernels_at_tile_edges(cuda, L, q, N):
     _lib.call("mi3_energies", dJ.data_ptr(), dm.data_ptr(), B, N, E.data_ptr(), L, q, ws.data_ptr(), ws.numel() * 8,
               stream())
     e64 = oracle.energies_f64(J, mem, L, q)[:N]
-    # float sums of <= 16 terms per row (2^-20 of the sum of magnitudes), the
-    # joint cells' and the final rounding
+    # a coupling is rounded in float 15 times at most (pair-major rows of 16),
+    # 4 to 6 times over joint sites: below 2^-20 of the sum of magnitudes; then
+    # the final rounding
     mag = oracle.energies_f64(np.abs(J), mem, L, q)[:N]
     assert np.all(np.abs(host(E) - e64) <= 2.0 ** -20 * mag + 2.0 ** -23 * np.abs(e64) + 1e-9)
 
@@ -62,7 +63,7 @@ def test_pair_kernels_at_tile_edges(cuda, L, q, N):
 
 
 @pytest.mark.parametrize("q", QS)
-@pytest.mark.parametrize("L", [33, 65])
+@pytest.mark.parametrize("L", [15, 31, 33, 65])
 def test_equal_sequences_have_equal_energies(cuda, L, q):
     """A sequence's energy depends on its residues alone, not on the lane or the
     chunk that sums it: copies tie, and share their average rank."""
