@@ -13,8 +13,15 @@ reseed, automatic equilibration of at least 64 sampler calls per round) and
 the carry-over schedule (walkers kept between rounds, one 2048-step call
 per round after an automatically equilibrated first round).  Tolerances:
 the SSR of the last rounds fluctuates by about +-30% from round to round
-(finite sampling), so the SSR must be below 0.015; Ferr within 10% and
-both X values within 0.6 of the quoted ones."""
+(finite sampling), so the SSR must be below 0.015; Ferr, the mean of the last
+12 rounds, within 10% and both X values within 0.6 of the quoted ones.
+
+Ferr of one round is no test: any change in how a float sum is rounded sends the
+rounds another way, and over six runs (two ways of adding energies, three seeds)
+the last 24 rounds spread by 6.7% about 0.0091, one in three of them more than
+10% off the quoted value.  Means of the last 12 rounds were 0.00876 to 0.00904
+in those runs, 2.3 to 5.6% above it, with a standard deviation of 1.2%: five of
+these below the bound."""
 from pathlib import Path
 
 import numpy as np
@@ -38,6 +45,7 @@ def test_hiv_example_reaches_reference_end_state(cuda, form):
     print(f"HIV {form}: SSR {last['ssr']:.4f} Ferr {last['ferr']:.5f} X {last['X']:.3f} ({last['Xo']:.3f}) "
           f"in {res['total_s']:.1f} s")
     assert last["ssr"] < 0.015, last
-    assert abs(last["ferr"] - float(fx["expect_ferr"])) < 0.1 * float(fx["expect_ferr"]), last
+    ferr = np.mean([h["ferr"] for h in res["history"][-12:]])
+    assert abs(ferr - float(fx["expect_ferr"])) < 0.1 * float(fx["expect_ferr"]), ferr
     assert abs(last["X"] - float(fx["expect_X"])) < 0.6, last
     assert abs(last["Xo"] - float(fx["expect_Xo"])) < 0.6, last
