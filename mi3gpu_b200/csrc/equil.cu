@@ -38,9 +38,10 @@ __device__ __forceinline__ uint32_t float_key(float x) {
 // (count[tile][digit], 1 KB per tile, read by every CTA from L2).  So a sort is
 // six launches, tie handling included, whatever n; the bitonic network it
 // replaces took 44 at n = 2^18, most of them 3 us long.  Call times, before and
-// now: 103 and 68 us at n = 2^14, 235 and 84 us at 2^18, 514 and 172 us at 2^20.
-// A pass is bound by its latencies: the reads of the counts, then 16 rounds of
-// matching.
+// now: 103 and 68 us at n = 2^14, 235 and 84 us at 2^18, 514 and 172 us at 2^20,
+// 3.5 and 2.7 ms at 2^23 - 1, where a pass reads 4 GB of counts from L2 (they grow
+// with n^2).  Below that a pass is bound by its latencies: the reads of the counts,
+// then 16 rounds of matching.
 constexpr uint32_t RK_THREADS = 256, RK_WARPS = RK_THREADS / 32, RK_PER = 16;
 constexpr uint32_t RK_TILE = RK_THREADS * RK_PER, RK_DIGITS = 256;
 

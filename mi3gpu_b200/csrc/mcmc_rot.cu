@@ -68,10 +68,22 @@
 // What bounds it (L=232, q=21): the shared-memory pipe (466 gathers per warp and
 // step plus the fill: 60% busy) and issue (75%) together, at 7 warps per
 // scheduler; 72 registers leave few loads in flight per warp.  Site-updates per
-// second of 2048-step-like calls, before (the faster of the two older kernels)
-// and now: L=48 q=4 2^14 1.4e10, 1.8e10; L=93 q=4 2^18 2.4e10, 6.0e10; L=187 q=8
-// 50688 1.0e10, 1.8e10; L=232 q=21 2^20 8.7e9, 1.16e10; L=512 q=21 2^18 3.2e9,
-// 3.7e9 (the fill: 0.9 MB of couplings per step for 448 walkers).
+// second of calls of 1 to 16 sweeps after new couplings, before (the faster of the
+// two older kernels) and now: L=48 q=4 2^14 2.9e10, 4.5e10; L=93 q=4 2^18 2.4e10,
+// 6.1e10; L=187 q=8 50688 9.8e9, 1.9e10; L=232 q=21 2^20 8.6e9, 1.18e10; L=512
+// q=21 2^18 3.2e9, 3.7e9 (the fill: 0.9 MB of couplings per step for 448 walkers).
+//
+// The couplings' size enters: the bound grows with them, and with a constant in
+// them that no dE contains, and an open verdict holds up its CTA for about 32 L
+// adds.  One sweep after new couplings N(0, s^2), in us (in brackets the older
+// kernel, which does not depend on them):
+//                      s=0.05   0.3     1      3    0.05 and 1 added  and 30 added
+//   L=93  q=4  2^18     517     517    518    523     522               668  [1248]
+//   L=187 q=8  50688    707     720    736    775     796              1629  [1459]
+//   L=232 q=21 2^18    5663    5825   6249   6938    7544             15713  [8317]
+//   L=400 q=21 2^16    6498    6628   7218   8223    9036             25681 [11718]
+// Couplings with such a constant are better re-gauged first
+// (mi3_gauge_fieldless_even leaves every dE as it is).
 #include <algorithm>
 #include <cmath>
 
