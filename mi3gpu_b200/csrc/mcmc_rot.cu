@@ -869,8 +869,8 @@ extern "C" uint64_t mi3_jrot_floats(uint32_t L, uint32_t q) {
 // Both models' errors are about 5%; where one lane can hold a walker's row, rot_cost
 // is the higher one by up to 20%, hence the tenth.  Beyond, q <= 4 never pays: the
 // row kernel's gathers mostly broadcast there.  Of 150 shapes the rotated kernel was
-// slower than the row kernel at ten before this test, by up to 37% (L=503, q=4,
-// 23552 walkers).
+// slower than the row kernel at ten before this test, taking up to 1.6 times as
+// long (L=503, q=4, 23552 walkers).
 extern "C" uint32_t mi3_metropolis_rot_pays(uint32_t L, uint32_t q, uint32_t nseqs) {
     RotShape r;
     if (!rot_shape(L, q, r) || nseqs == 0 || nseqs % 32) return 0;
